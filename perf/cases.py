@@ -26,7 +26,7 @@ import torch
 
 from cleo_b200 import abi
 from cleo_b200 import workloads as W
-from cleo_b200.config import (COORD0, LLIM, MR0, Mr_ratio, Mr_sol, P0, R0, RHO0, Rho_sol, TEMP0,
+from cleo_b200.config import (LLIM, MR0, Mr_ratio, Mr_sol, P0, R0, RHO0, Rho_sol, TEMP0,
                               TIME0, VOL0, cartesian_grid, make_params)
 from cleo_b200.sdm import SDM, CleoError
 from cleo_b200.surrogate import Surrogate, condensation_solve, train_surrogate
