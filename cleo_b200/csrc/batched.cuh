@@ -266,36 +266,24 @@ k_cond_a(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch 
         // the condensate mass qcond sums (k_b_qcond's term), for the commit to add in order
         if (b.qm) b.qm[i] = condensate_mass(r, msol, w) * (double)c.sd.xi[i];
         const double ffactor_fv = b.th_ff[g] / ventilation_factor(r);
-        const OdeConsts o{b.th_s[g], b.th_ak[g], kohler_b(msol), ffactor_fv};
+        const OdeConsts o = ode_consts(b.th_s[g], b.th_ak[g], kohler_b(msol), ffactor_fv);
         const double z0 = initialguess_a3(o, r, b.th_a3[g]);
         // ucrit1 || ucrit2, the critical timestep only evaluated when ucrit1 fails
         const bool ucrit1 = first_unique_a3(o, r, z0, b.th_u3[g]);
         double crit = 0.0;
         uint32_t ni = 0;
         if (ucrit1 || below_critical_timestep(o, p.cond_delt, crit)) {
-          bool conv = false, conv1 = false;
-          double z1 = 0.0;
-          GEval e = eval_g(o, p.cond_delt, r, z0);
-#pragma unroll 1
-          for (int it = 0; it < 2; ++it) {  // one copy of the iteration: a smaller hot loop
-            e = nr_iterate(cfg, o, p.cond_delt, r, e, conv, ni);
-            if (it == 0) {
-              conv1 = conv;
-              z1 = e.z;
-            }
-          }
-          if (!conv) {
-            b.zres[i] = conv1 ? -z1 : e.z;  // where pass B's restart continues
+          double radius, zres;
+          if (!two_iterations(cfg, o, p.cond_delt, r, z0, ni, radius, zres)) {
+            defer = true;  // restart from z0 until converged (impliciteuler.cpp:136-140)
+            b.zres[i] = zres;
             b.ffv[i] = ffactor_fv;
-          }
-          if (conv) {
-            const double rnew = max_dryradius(sqrt(e.z), msol);  // change_radius
+          } else {
+            const double rnew = max_dryradius(radius, msol);  // change_radius
             b.dm[i] = (condensate_mass(rnew, msol, w) - condensate_mass(r, msol, w)) *
                       (double)c.sd.xi[i];
             b.its[i] = ni;
             c.sd.r[i] = rnew;
-          } else {
-            defer = true;  // restart from z0 until converged (impliciteuler.cpp:136-140)
           }
         } else {
           defer = true;
@@ -339,16 +327,15 @@ k_cond_b(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch 
     if (b.lkeys[j] == 0u && cfg.maxniters >= 2) {
       // a direct solve whose two iterations in pass A did not converge: the restart continues
       // from them (resume_restart), unless the surrogate's seed converges first
-      const OdeConsts o{b.th_s[g], akoh, bkoh, b.ffv[i]};  // pass A's th_ff / ventilation
+      const OdeConsts o = ode_consts(b.th_s[g], akoh, bkoh, b.ffv[i]);  // pass A's th_ff / ventilation
       ni = 2;
       double rsqrd = 0.0;
       bool done = false;
       if (seed_ok(seed)) {
         const double z0 = initialguess_a3(o, r, b.th_a3[g]);
         const bool ucrit1 = first_unique_a3(o, r, z0, b.th_u3[g]);
-        const GEval e0 = eval_g(o, p.cond_delt, r, z0);
-        const GEval es = eval_g(o, p.cond_delt, r, seed);
-        done = fabs(es.g) < fabs(e0.g) && integrate_seeded(cfg, o, p.cond_delt, r, es, ni, rsqrd) &&
+        bool tried;
+        done = integrate_seeded(cfg, o, p.cond_delt, r, z0, seed, ni, rsqrd, tried) &&
                seeded_root_ok(o, ucrit1, rsqrd);
       }
       if (!done) {

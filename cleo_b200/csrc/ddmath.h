@@ -428,4 +428,56 @@ CLEO_MATH_HD void dpow2(double x, double y1, double y2, double& p1, double& p2) 
   p2 = out[1];
 }
 
+// ---- quotients and square roots that share a reciprocal ----
+// The Newton iteration of condensation divides by the same few numbers again and again (r, r^3,
+// z F). With y = RN(1 / b) at hand, P. Markstein's correction (IBM J. Res. Dev. 34 (1990)
+// 111-119) gives the IEEE quotient a / b in three operations without a branch: q = RN(a y) is
+// within 1.5 ulp, its residual a - b q is (all but) exact in one fused multiply-add, and
+// RN(q + (a - b q) y) has an error of 2^-51 ulp before its rounding, so it is the correctly
+// rounded quotient unless a / b lies that near a rounding boundary. Operands stay within
+// in_window, so nothing over- or underflows. The one divisor whose reciprocal polishing does not
+// round right is the significand of all ones (all_ones): it lies 2^-54 past a midpoint.
+CLEO_MATH_HD double quot(double a, double b, double y) {
+  const double q = a * y;
+  return dd_fma(dd_fma(-b, q, a), y, q);
+}
+CLEO_MATH_HD bool all_ones(double b) {
+  const uint64_t u = dbits(b);
+  return (((uint32_t)(u >> 32) | 0xFFF00000u) & (uint32_t)u) == 0xFFFFFFFFu;
+}
+// RN(1 / b) from y within a few ulp of it (the error squares, to 2^-100, before the rounding)
+CLEO_MATH_HD double recip_polish(double b, double y) {
+  return dd_fma(dd_fma(-b, y, 1.0), y, y);
+}
+// RN(1 / b) from a first y with a relative error up to 2^-19: a cubic step (to 2^-55), polished.
+// b of all ones, 2^k (2 - 2^-52) (the derivative of a residual, 1 less a tiny product, is one):
+// 1 / b = 2^-(k+1) (1 + 2^-53 + ...), rounded to 2^-(k+1) (1 + 2^-52), put together from its bits.
+CLEO_MATH_HD double recip_from(double b, double y) {
+  double e = dd_fma(-b, y, 1.0);
+  e = dd_fma(e, e, e);
+  const double r = recip_polish(b, dd_fma(y, e, y));
+  const uint64_t u = dbits(b);
+  const uint64_t ones = (u & 0x8000000000000000ull) |
+                        ((uint64_t)(2045u - ((uint32_t)(u >> 52) & 0x7FFu)) << 52) | 1ull;
+  return all_ones(b) ? bitsd(ones) : r;
+}
+// s = RN(sqrt(z)) and y = RN(1 / s) from a first y for 1 / sqrt(z) with a relative error up to
+// 2^-19: a cubic step y (1 + e / 2 + 3 e^2 / 8), e = 1 - z y^2 (to 2^-52 with its roundings);
+// s0 = z y corrected by its exact residual, (z - s0^2) y / 2, an error of 2^-51 ulp before the
+// rounding. sqrt(z) lies that near a midpoint only for a handful of significands z (M^2 + M + k
+// for k = 0 and 2), which the tests go through.
+CLEO_MATH_HD void sqrt_recip_from(double z, double y, double& s, double& yr) {
+  const double e = dd_fma(-(z * y), y, 1.0);
+  y = dd_fma(y * e, dd_fma(e, 0.375, 0.5), y);
+  const double s0 = z * y;
+  s = dd_fma(dd_fma(-s0, s0, z), 0.5 * y, s0);
+  yr = recip_polish(s, y);
+}
+// x positive with its exponent in [-150, 150): products, quotients and residuals of a few such
+// numbers are normal doubles
+CLEO_MATH_HD bool in_window(double x) {
+  const uint32_t hi = (uint32_t)(dbits(x) >> 32);
+  return hi - ((1023u - 150u) << 20) < (300u << 20);
+}
+
 }  // namespace cleo

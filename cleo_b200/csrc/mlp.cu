@@ -75,7 +75,7 @@ __global__ void k_mlp_features(uint32_t n, const double* __restrict__ radius,
       const double ffactor = diffusion_factor(press[i], T, psat);
       double akoh, bkoh;
       kohler_factors(msol[i], T, akoh, bkoh);
-      const OdeConsts o{s_ratio[i], akoh, bkoh, ffactor / ventilation_factor(radius[i])};
+      const OdeConsts o = ode_consts(s_ratio[i], akoh, bkoh, ffactor / ventilation_factor(radius[i]));
       const double z0 = initialguess(o, radius[i]);
       direct[i] = (first_unique_criteria(o, radius[i], z0) || delt[i] <= critical_timestep(o))
                       ? 1

@@ -488,6 +488,24 @@ __device__ __forceinline__ double ventilation_factor_cr(double radius) {
   const double vent_factor = 1.0 + 1.0 / (a + b);
   return fmin(vent_factor, vent_factor_max);
 }
+// first approximations of 1 / b and 1 / sqrt(z) (relative error about 2^-20), refined by the caller
+__device__ __forceinline__ double rcp_seed(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  return y;
+}
+__device__ __forceinline__ double rsqrt_seed(double z) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(z));
+  return y;
+}
+// 1 / b to a relative 2^-52 (in_window b), where the last bit does not matter
+__device__ __forceinline__ double recip_near(double b) {
+  const double y = rcp_seed(b);
+  double e = dd_fma(-b, y, 1.0);
+  e = dd_fma(e, e, e);
+  return dd_fma(y, e, y);
+}
 // x^y for 2^-60 <= x < 1 (x = 2^e m, m in [1, 2)) from the library's log2 and exp2, relative
 // error below 2^-50: log2 m to 2^-53 absolute (1 ulp documented, |log2 m| < 1), so y log2 m to
 // 2^-51 with its rounding (y < 2); y e exact as a double-double; exp2 of the sum's high part
@@ -515,9 +533,9 @@ __device__ __forceinline__ double ventilation_factor(double radius) {
     const int e = (int)((xb >> 52) & 0x7FF) - 1023;
     const double lm = log2(bitsd((xb & 0x000FFFFFFFFFFFFFull) | 0x3FF0000000000000ull));
     const double pa = vent_pow(1.963, e, lm), pb = vent_pow(0.702, e, lm);
-    const double a = 1.0 / (6.954e+7 * pa);
-    const double b = 1.0 / (1.069e+3 * pb);
-    const double d = 1.0 / (a + b);
+    const double a = recip_near(6.954e+7 * pa);
+    const double b = recip_near(1.069e+3 * pb);
+    const double d = recip_near(a + b);
     const dd v = two_sum(1.0, d);  // v.hi = RN(1 + d), v.lo = 1 + d - v.hi exactly
     const double bound = d * 0x1p-47;
     const uint64_t vb = dbits(v.hi);
@@ -534,7 +552,9 @@ __device__ __forceinline__ double kohler_a(double temp) {
 }
 __device__ __forceinline__ double kohler_b(double msol) {
   const double bkoh_constant = 4.3e-6 * RHO0 / MR0;
-  return bkoh_constant * msol * IONIC / Mr_sol;
+  const double x = bkoh_constant * msol * IONIC;
+  if (in_window(x)) return quot(x, Mr_sol, 1.0 / Mr_sol);  // (the constant's reciprocal is exact)
+  return x / Mr_sol;
 }
 __device__ __forceinline__ void kohler_factors(double msol, double temp, double& akoh,
                                                double& bkoh) {
@@ -543,9 +563,19 @@ __device__ __forceinline__ void kohler_factors(double msol, double temp, double&
 }
 
 // ---- ImplicitEuler: impliciteuler.{hpp:41-345, cpp:35-301} ----
+// The droplet's constants of one solve; yf = 1 / ffactor_fv. `fast` where all of them are
+// in_window: the solve may then use shared reciprocals.
 struct OdeConsts {
-  double s_ratio, akoh, bkoh, ffactor_fv;
+  double s_ratio, akoh, bkoh, ffactor_fv, yf;
+  bool fast;
 };
+__device__ __forceinline__ OdeConsts ode_consts(double s_ratio, double akoh, double bkoh,
+                                                double ffactor_fv) {
+  OdeConsts o{s_ratio, akoh, bkoh, ffactor_fv, 0.0, false};
+  o.fast = in_window(akoh) && in_window(ffactor_fv) && (bkoh == 0.0 || in_window(bkoh));
+  o.yf = recip_from(ffactor_fv, rcp_seed(ffactor_fv));
+  return o;
+}
 struct NewtonCfg {
   uint32_t maxniters;
   double rtol, atol;
@@ -563,84 +593,227 @@ constexpr uint32_t NR_ITER_CAP = 4u << 20;
 // g's beta is (2 subdelt) / (z F) and g''s is subdelt / (z F) with the same rounded product z F;
 // scaling by 2 commutes with rounding to nearest (no overflow or underflow at these magnitudes),
 // so the first is exactly twice the second and one division serves both.
+//
+// What bounds it: FP64 issue, and in the long sub-stepping solves the latency of one iteration's
+// chain. Four of the six divisions of an iteration share a divisor's reciprocal, and those
+// reciprocals follow from the one of the root: 1/r from the square root's own start, 1/r^3 and
+// 1/(z F) from products of it, each polished in two operations, each quotient then three (quot).
+// The compiler's division and square root carry a branch each, which also keeps independent ones
+// from overlapping; the FAST form has none. It adds up in `bad` what it cannot answer for
+// (operands out of in_window, r, r^3 or z F all_ones); the solve is then repeated with the
+// operators (FAST = false), which a sound run meets once in some 10^15 evaluations.
 struct GEval {
-  double z, radius, akr, r3, q, g;
+  double z, radius, akr, r3, y3, alpha, q, g;  // y3: RN(1 / r3), in the FAST form
 };
+template <bool FAST>
 __device__ __forceinline__ GEval eval_g(const OdeConsts& o, double subdelt, double rprev,
-                                        double rsqrd) {
+                                        double rsqrd, bool& bad) {
   GEval e;
   e.z = rsqrd;
-  e.radius = sqrt(rsqrd);
-  e.akr = o.akoh / e.radius;
-  e.r3 = dpow(e.radius, 3.0);
-  const double alpha = o.s_ratio - 1 - e.akr + o.bkoh / e.r3;
-  e.q = subdelt / (rsqrd * o.ffactor_fv);
-  const double beta = 2.0 * e.q;
-  const double gamma = dpow(rprev / e.radius, 2.0);
-  e.g = 1 - gamma - alpha * beta;
+  if constexpr (FAST) {
+    double yr;
+    sqrt_recip_from(rsqrd, rsqrt_seed(rsqrd), e.radius, yr);
+    const double y2 = yr * yr;
+    const double zf = rsqrd * o.ffactor_fv;
+    e.akr = quot(o.akoh, e.radius, yr);
+    // r^3 rounded once (dpow's exact square and product; their sum's rounding is the result)
+    const dd x2 = two_prod(e.radius, e.radius);
+    const dd x3 = two_prod(x2.hi, e.radius);
+    e.r3 = x3.hi + (x3.lo + x2.lo * e.radius);
+    e.y3 = recip_polish(e.r3, y2 * yr);
+    e.alpha = o.s_ratio - 1 - e.akr + quot(o.bkoh, e.r3, e.y3);
+    e.q = quot(subdelt, zf, recip_polish(zf, y2 * o.yf));
+    const double ratio = quot(rprev, e.radius, yr);
+    // 1 - gamma - alpha beta, beta = 2 q: doubling is exact, so one fused operation subtracts the
+    // rounded product as the reference does
+    e.g = dd_fma(-2.0, e.alpha * e.q, 1 - ratio * ratio);
+    bad = bad | !in_window(rsqrd) | all_ones(e.radius) | all_ones(e.r3) | all_ones(zf);
+  } else {
+    e.radius = sqrt(rsqrd);
+    e.akr = o.akoh / e.radius;
+    e.r3 = dpow(e.radius, 3.0);
+    e.y3 = 0.0;
+    e.alpha = o.s_ratio - 1 - e.akr + o.bkoh / e.r3;
+    e.q = subdelt / (rsqrd * o.ffactor_fv);
+    const double gamma = dpow(rprev / e.radius, 2.0);
+    e.g = 1 - gamma - e.alpha * (2.0 * e.q);
+  }
   return e;
 }
-__device__ __forceinline__ double eval_gprime(const OdeConsts& o, const GEval& e) {
-  const double alpha = e.akr - 3.0 * o.bkoh / e.r3;
-  return 1 - alpha * e.q;
+// whether the FAST form may start from these: the first iterate checks itself
+__device__ __forceinline__ bool fast_start(const OdeConsts& o, double subdelt, double rprev) {
+  return o.fast && in_window(subdelt) && in_window(rprev);
+}
+// ode_gfuncderivative (:291-301) at e, with its reciprocal in the FAST form
+struct GPrime {
+  double den, y;
+};
+template <bool FAST>
+__device__ __forceinline__ GPrime eval_gprime(const OdeConsts& o, const GEval& e, bool& bad) {
+  GPrime d{0.0, 0.0};
+  const double b3 = 3.0 * o.bkoh;
+  if constexpr (FAST) {
+    d.den = 1 - (e.akr - quot(b3, e.r3, e.y3)) * e.q;
+    d.y = recip_from(d.den, rcp_seed(d.den));
+    bad = bad | !in_window(fabs(d.den));
+  } else {
+    d.den = 1 - (e.akr - b3 / e.r3) * e.q;
+  }
+  return d;
 }
 // iterate_rootfinding_algorithm: impliciteuler.cpp:239-255 (+ check_for_convergence, hpp:213-219)
+template <bool FAST>
 __device__ __forceinline__ GEval nr_iterate(const NewtonCfg& c, const OdeConsts& o,
                                             double subdelt, double rprev, const GEval& e,
-                                            bool& converged, uint32_t& niters) {
-  const double numerator = e.g;
-  const double denominator = eval_gprime(o, e);
-  double ziter = e.z * (1 - numerator / denominator);
+                                            const GPrime& d, bool& converged, uint32_t& niters,
+                                            bool& bad) {
+  const double num = e.g;
+  double step;
+  if constexpr (FAST) {
+    step = quot(num, d.den, d.y);
+    bad = bad | !((num == 0.0) | in_window(fabs(num)));
+  } else {
+    step = num / d.den;
+  }
+  double ziter = e.z * (1 - step);
   ziter = fmax(ziter, 1e-8);
-  const GEval next = eval_g(o, subdelt, rprev, ziter);
+  const GEval next = eval_g<FAST>(o, subdelt, rprev, ziter, bad);
   const double conv = c.rtol * fabs(next.g) + c.atol;
-  converged = fabs(next.g - numerator) < conv;
+  converged = fabs(next.g - num) < conv;
   ++niters;
   return next;
 }
-// integrate_condensation_ode: impliciteuler.cpp:128-141 with newtonraphson_niterations (:181-194)
-// and newtonraphson_untilconverged (:207-227). e0 is g at the initial guess. Returns 0 or the
-// failure code; z receives the last iterate either way.
-__device__ __forceinline__ int integrate_ode_core(const NewtonCfg& c, const OdeConsts& o,
-                                                  double subdelt, double rprev, const GEval& e0,
-                                                  uint32_t& niters, double& z) {
+template <bool FAST>
+__device__ __forceinline__ GEval nr_iterate(const NewtonCfg& c, const OdeConsts& o,
+                                            double subdelt, double rprev, const GEval& e,
+                                            bool& converged, uint32_t& niters, bool& bad) {
+  const GPrime d = eval_gprime<FAST>(o, e, bad);
+  return nr_iterate<FAST>(c, o, subdelt, rprev, e, d, converged, niters, bad);
+}
+
+// The sub-steps of a solve (:98-113) as one loop of Newton iterations: a lane that has finished a
+// sub-step starts its next one in the same pass, so a warp takes as many passes as its longest
+// solve has iterations, not the sum over sub-steps of each one's longest. The vote keeps the
+// warp's lanes together whatever phase each is in. A sub-step is integrate_condensation_ode
+// (:128-141) with newtonraphson_niterations (:181-194) and newtonraphson_untilconverged
+// (:207-227): two iterations; if the second did not converge, the restart from the sub-step's
+// first iterate, whose first two iterations repeat them exactly and are taken from them, each
+// behind the checks the restart makes before it. A direct solve is one sub-step of delt.
+// Returns the last iterate; `code` keeps the first failure.
+template <bool FAST>
+__device__ __forceinline__ double newton_solve(const NewtonCfg& c, const OdeConsts& o, double delt,
+                                               double mindelt, double rprev, double z0,
+                                               bool direct, uint32_t& niters, int& code,
+                                               bool& bad) {
+  double remdelt = delt, subdelt = fmin(mindelt, delt);
+  double z = z0, z1 = 0.0;
+  bool conv1 = false;
+  uint32_t k = 0;  // iterations of this sub-step
+  bool run = direct || remdelt > 0.0;  // a direct solve whatever its time step
+  if constexpr (FAST) {
+    if (!fast_start(o, subdelt, rprev)) bad = true;
+  }
+  GEval e = eval_g<FAST>(o, subdelt, rprev, z0, bad);
+  // g' and its reciprocal are taken with g, before the tests on g: the two chains overlap, and the
+  // next sub-step's first iteration, at the same z, needs the same g'
+  GPrime d = eval_gprime<FAST>(o, e, bad);
+  const unsigned lanes = __activemask();
+  while (__any_sync(lanes, run)) {
+    if (run) {
+      bool conv;
+      const bool first = k == 0;
+      z0 = first ? e.z : z0;
+      e = nr_iterate<FAST>(c, o, subdelt, rprev, e, d, conv, niters, bad);
+      d = eval_gprime<FAST>(o, e, bad);
+      ++k;
+      z = e.z;
+      z1 = first ? z : z1;
+      conv1 = first ? conv : conv1;
+      bool ended = conv & !first;
+      if (!(conv | first) | bad) {
+        int f = 0;
+        if (k == 2) {  // the repeated iterations: zr what the restart would return at this point
+          double zr = z0;
+          if (1 > c.maxniters) {
+            f = CLEO_ERR_NR_NOCONVERGE;
+          } else if (niters >= NR_ITER_CAP) {
+            f = CLEO_ERR_TIMEOUT;
+          } else {
+            ++niters;
+            zr = z1;
+            if (conv1) {
+              ended = true;
+            } else if (2 > c.maxniters) {
+              f = CLEO_ERR_NR_NOCONVERGE;
+            } else if (niters >= NR_ITER_CAP) {
+              f = CLEO_ERR_TIMEOUT;
+            } else {
+              ++niters;
+              zr = z;
+            }
+          }
+          z = zr;
+        }
+        if (f == 0 && !ended) {
+          if (k + 1 > c.maxniters)
+            f = CLEO_ERR_NR_NOCONVERGE;
+          else if (niters >= NR_ITER_CAP)
+            f = CLEO_ERR_TIMEOUT;
+        }
+        if (f) {
+          if (code == 0) code = f;
+          ended = true;
+        }
+        if (FAST && bad) ended = run = false;
+      }
+      if (ended) {
+        remdelt -= subdelt;
+        k = 0;
+        const double next = fmin(mindelt, remdelt);
+        if (FAST & (next == subdelt) & (z == e.z) & (niters < NR_ITER_CAP) & !direct) {
+          // the same time step from the last iterate: r_prev = sqrt(z) is its radius, so gamma is
+          // exactly 1; all else of g, and g', stays
+          rprev = e.radius;
+          e.g = dd_fma(-2.0, e.alpha * e.q, 0.0);
+        } else {
+          run = !direct && remdelt > 0.0;
+          if (run && niters >= NR_ITER_CAP) {
+            if (code == 0) code = CLEO_ERR_TIMEOUT;
+            run = false;
+          }
+          if (run) {
+            subdelt = next;
+            rprev = sqrt(z);
+            e = eval_g<FAST>(o, subdelt, rprev, z, bad);
+            d = eval_gprime<FAST>(o, e, bad);
+          }
+        }
+      }
+    }
+  }
+  return z;
+}
+// The restart of a sub-step when the two iterations before it have already been done: it
+// continues from them. zres is -z1 when the first iteration passed the convergence test (the
+// restart stops after it) and z2 otherwise (the second did not pass it, or there would be no
+// restart). Adds the restart's iterations, the repeated ones included, to niters; needs
+// maxniters >= 2.
+template <bool FAST>
+__device__ __forceinline__ double resume_restart_as(const NewtonCfg& c, const OdeConsts& o,
+                                                    double subdelt, double rprev, double zres,
+                                                    uint32_t& niters, int& code, bool& bad) {
+  if (zres < 0.0) {
+    niters += 1;
+    return -zres;
+  }
+  niters += 2;
+  if constexpr (FAST) {
+    if (!fast_start(o, subdelt, rprev)) bad = true;
+  }
+  GEval e = eval_g<FAST>(o, subdelt, rprev, zres, bad);
   bool conv = false;
-  GEval e = nr_iterate(c, o, subdelt, rprev, e0, conv, niters);
-  const bool conv1 = conv;
-  const double z1 = e.z;
-  e = nr_iterate(c, o, subdelt, rprev, e, conv, niters);
-  if (conv) {
-    z = e.z;
-    return 0;
-  }
-  // the restart from e0 (newtonraphson_untilconverged): its first two iterations repeat the two
-  // above exactly, so they are taken from them, each behind the checks the restart makes before it
-  if (1 > c.maxniters) {
-    z = e0.z;
-    return CLEO_ERR_NR_NOCONVERGE;
-  }
-  if (niters >= NR_ITER_CAP) {
-    z = e0.z;
-    return CLEO_ERR_TIMEOUT;
-  }
-  niters += 1;
-  if (conv1) {
-    z = z1;
-    return 0;
-  }
-  if (2 > c.maxniters) {
-    z = z1;
-    return CLEO_ERR_NR_NOCONVERGE;
-  }
-  if (niters >= NR_ITER_CAP) {
-    z = z1;
-    return CLEO_ERR_TIMEOUT;
-  }
-  niters += 1;
-  conv = false;  // as after the second iteration above
   uint32_t niter = 3;
-  int code = 0;
-  while (!conv) {
+  while (!conv && !(FAST && bad)) {
     if (niter > c.maxniters) {
       code = CLEO_ERR_NR_NOCONVERGE;
       break;
@@ -649,53 +822,40 @@ __device__ __forceinline__ int integrate_ode_core(const NewtonCfg& c, const OdeC
       code = CLEO_ERR_TIMEOUT;
       break;
     }
-    e = nr_iterate(c, o, subdelt, rprev, e, conv, niters);
+    e = nr_iterate<FAST>(c, o, subdelt, rprev, e, conv, niters, bad);
     niter += 1;
   }
-  z = e.z;
-  return code;
+  return e.z;
 }
-// The restart of integrate_ode_core (newtonraphson_untilconverged from the initial guess,
-// impliciteuler.cpp:131-132, 207-227) when the two iterations before it have already been done:
-// the restart's first two iterations repeat them exactly, so it can continue from them. zres is
-// -z1 when the first iteration passed the convergence test (the restart stops after it) and z2
-// otherwise (the second did not pass it, or there would be no restart). Adds the restart's
-// iterations, the repeated ones included, to niters; needs maxniters >= 2.
+// the two above with the operators, for the solves the FAST form gives up
+static __device__ __noinline__ double newton_solve_wide(const NewtonCfg& c, const OdeConsts& o,
+                                                        double delt, double mindelt, double rprev,
+                                                        double z0, bool direct, uint32_t& niters,
+                                                        int& code) {
+  bool unused = false;
+  return newton_solve<false>(c, o, delt, mindelt, rprev, z0, direct, niters, code, unused);
+}
+static __device__ __noinline__ double resume_restart_wide(const NewtonCfg& c, const OdeConsts& o,
+                                                          double subdelt, double rprev,
+                                                          double zres, uint32_t& niters,
+                                                          int& code) {
+  bool unused = false;
+  return resume_restart_as<false>(c, o, subdelt, rprev, zres, niters, code, unused);
+}
 __device__ __forceinline__ int resume_restart(const NewtonCfg& c, const OdeConsts& o,
                                               double subdelt, double rprev, double zres,
                                               uint32_t& niters, double& z) {
-  if (zres < 0.0) {
-    niters += 1;
-    z = -zres;
-    return 0;
-  }
-  niters += 2;
-  GEval e = eval_g(o, subdelt, rprev, zres);
-  bool conv = false;
-  uint32_t niter = 3;
+  bool bad = false;
   int code = 0;
-  while (!conv) {
-    if (niter > c.maxniters) {
-      code = CLEO_ERR_NR_NOCONVERGE;
-      break;
-    }
-    if (niters >= NR_ITER_CAP) {
-      code = CLEO_ERR_TIMEOUT;
-      break;
-    }
-    e = nr_iterate(c, o, subdelt, rprev, e, conv, niters);
-    niter += 1;
+  uint32_t n = niters;
+  z = resume_restart_as<true>(c, o, subdelt, rprev, zres, n, code, bad);
+  if (bad) {
+    n = niters;
+    code = 0;
+    z = resume_restart_wide(c, o, subdelt, rprev, zres, n, code);
   }
-  z = e.z;
+  niters = n;
   return code;
-}
-__device__ __forceinline__ double integrate_ode(const NewtonCfg& c, const OdeConsts& o,
-                                                double subdelt, double rprev, const GEval& e0,
-                                                uint32_t& niters, const Where& w) {
-  double z;
-  const int code = integrate_ode_core(c, o, subdelt, rprev, e0, niters, z);
-  if (code) w.fail(code);
-  return z;
 }
 // a usable seed: finite and positive (NaN compares false)
 __device__ __forceinline__ bool seed_ok(double seed_rsqrd) {
@@ -703,17 +863,45 @@ __device__ __forceinline__ bool seed_ok(double seed_rsqrd) {
 }
 // Newton iterations from a seed, the convergence test (check_for_convergence) after every one,
 // at most SEED_MAXITERS: a good seed converges in one or two, a poor one is abandoned early
-// (the caller then starts from the reference guess). Returns true when converged.
+// (the caller then starts from the reference guess). Returns true when converged. The seed is
+// tried when its residual is smaller than the reference guess's, g0; tried reports that.
 constexpr uint32_t SEED_MAXITERS = 6;
-__device__ __forceinline__ bool integrate_seeded(const NewtonCfg& c, const OdeConsts& o,
-                                                 double subdelt, double rprev, GEval e,
-                                                 uint32_t& niters, double& z) {
-  bool conv = false;
-  for (uint32_t k = 0; k < SEED_MAXITERS; ++k) {
-    e = nr_iterate(c, o, subdelt, rprev, e, conv, niters);
-    if (conv) break;
+template <bool FAST>
+__device__ __forceinline__ bool seeded_as(const NewtonCfg& c, const OdeConsts& o, double subdelt,
+                                          double rprev, double z0, double seed, uint32_t& niters,
+                                          double& z, bool& tried, bool& bad) {
+  if constexpr (FAST) {
+    if (!fast_start(o, subdelt, rprev)) bad = true;
   }
+  const GEval e0 = eval_g<FAST>(o, subdelt, rprev, z0, bad);
+  GEval e = eval_g<FAST>(o, subdelt, rprev, seed, bad);
+  bool conv = false;
+  tried = fabs(e.g) < fabs(e0.g);
+  if (tried)
+    for (uint32_t k = 0; k < SEED_MAXITERS && !conv; ++k)
+      e = nr_iterate<FAST>(c, o, subdelt, rprev, e, conv, niters, bad);
   z = e.z;
+  return conv;
+}
+static __device__ __noinline__ bool seeded_wide(const NewtonCfg& c, const OdeConsts& o,
+                                                double subdelt, double rprev, double z0,
+                                                double seed, uint32_t& niters, double& z,
+                                                bool& tried) {
+  bool unused = false;
+  return seeded_as<false>(c, o, subdelt, rprev, z0, seed, niters, z, tried, unused);
+}
+__device__ __forceinline__ bool integrate_seeded(const NewtonCfg& c, const OdeConsts& o,
+                                                 double subdelt, double rprev, double z0,
+                                                 double seed, uint32_t& niters, double& z,
+                                                 bool& tried) {
+  bool bad = false;
+  uint32_t n = niters;
+  bool conv = seeded_as<true>(c, o, subdelt, rprev, z0, seed, n, z, tried, bad);
+  if (bad) {
+    n = niters;
+    conv = seeded_wide(c, o, subdelt, rprev, z0, seed, n, z, tried);
+  }
+  niters = n;
   return conv;
 }
 // Whether a root reached from a seed is the root the reference's guess leads to. With
@@ -725,15 +913,77 @@ __device__ __forceinline__ bool integrate_seeded(const NewtonCfg& c, const OdeCo
 __device__ __forceinline__ bool seeded_root_ok(const OdeConsts& o, bool ucrit1, double z) {
   return !ucrit1 || z <= 3.0 * o.bkoh / o.akoh;
 }
+// The first two iterations of a direct solve from z0 (pass A): whether the second converged, with
+// the radius of its iterate; else zres for the restart (resume_restart).
+template <bool FAST>
+__device__ __forceinline__ bool two_iterations_as(const NewtonCfg& c, const OdeConsts& o,
+                                                  double delt, double rprev, double z0,
+                                                  uint32_t& niters, double& radius, double& zres,
+                                                  bool& bad) {
+  bool conv = false, conv1 = false;
+  double z1 = 0.0;
+  if constexpr (FAST) {
+    if (!fast_start(o, delt, rprev)) bad = true;
+  }
+  GEval e = eval_g<FAST>(o, delt, rprev, z0, bad);
+#pragma unroll 1
+  for (int it = 0; it < 2; ++it) {  // one copy of the iteration: a smaller hot loop
+    e = nr_iterate<FAST>(c, o, delt, rprev, e, conv, niters, bad);
+    if (it == 0) {
+      conv1 = conv;
+      z1 = e.z;
+    }
+  }
+  radius = e.radius;
+  zres = conv1 ? -z1 : e.z;
+  return conv;
+}
+static __device__ __noinline__ bool two_iterations_wide(const NewtonCfg& c, const OdeConsts& o,
+                                                        double delt, double rprev, double z0,
+                                                        uint32_t& niters, double& radius,
+                                                        double& zres) {
+  bool unused = false;
+  return two_iterations_as<false>(c, o, delt, rprev, z0, niters, radius, zres, unused);
+}
+__device__ __forceinline__ bool two_iterations(const NewtonCfg& c, const OdeConsts& o, double delt,
+                                               double rprev, double z0, uint32_t& niters,
+                                               double& radius, double& zres) {
+  bool bad = false;
+  uint32_t n = niters;
+  bool conv = two_iterations_as<true>(c, o, delt, rprev, z0, n, radius, zres, bad);
+  if (bad) {
+    n = niters;
+    conv = two_iterations_wide(c, o, delt, rprev, z0, n, radius, zres);
+  }
+  niters = n;
+  return conv;
+}
 // The factors of initialguess and first_unique_criteria that depend on akoh alone, i.e. on the
 // gridbox's temperature: the batched schedule evaluates them once per gridbox (same expressions,
 // so the same doubles). The two differ in rounding (a correctly rounded cube against a product).
 __device__ __forceinline__ double activation_a3(double akoh) { return 4.0 * dpow(akoh, 3.0) / 27; }
 __device__ __forceinline__ double unique_a3(double akoh) { return 4.0 * akoh * akoh * akoh / 27.0; }
+// s_ratio against 1 + sqrt(a3 / bkoh), decided without the division and the root where they cannot
+// matter: not above 1 it never exceeds the sum; above, s - 1 is exact, and (s - 1)^2 bkoh outside
+// a band of 1e-9 around a3 decides, while the root is above 1e-5 (the sum's rounding, 2^-52 and
+// what a3's two roundings and the operations add, moves the root by far less). Returns the sign of
+// s_ratio - sum: 1 above, -1 not above; both of the reference's comparisons follow from it.
+__device__ __forceinline__ int activation_side(double s_ratio, double bkoh, double a3) {
+  const double u = s_ratio - 1.0;
+  if (bkoh >= 0.0 && a3 >= 0.0) {
+    if (u <= 0.0) return -1;
+    const double lhs = u * u * bkoh;
+    if (a3 > 1e-10 * bkoh && a3 <= DBLMAX) {
+      if (lhs > a3 * (1.0 + 1e-9)) return 1;
+      if (lhs < a3 * (1.0 - 1e-9)) return -1;
+    }
+  }
+  return 0;  // not decided
+}
 // initialguess (:156-170) given a3 = activation_a3(o.akoh)
 __device__ __forceinline__ double initialguess_a3(const OdeConsts& o, double rprev, double a3) {
-  const double s_act = 1 + sqrt(a3 / o.bkoh);
-  if (o.s_ratio > s_act) {
+  const int side = activation_side(o.s_ratio, o.bkoh, a3);
+  if (side != 0 ? side > 0 : o.s_ratio > 1 + sqrt(a3 / o.bkoh)) {
     const double bigr = 1e-3 / R0;
     const double maxradius = fmax(bigr, rprev);
     return maxradius * maxradius;
@@ -743,17 +993,24 @@ __device__ __forceinline__ double initialguess_a3(const OdeConsts& o, double rpr
 __device__ __forceinline__ double initialguess(const OdeConsts& o, double rprev) {  // :156-170
   return initialguess_a3(o, rprev, activation_a3(o.akoh));
 }
+// z < 3 bkoh / akoh, by z akoh against 3 bkoh outside a band of 1e-12 (each side rounds by a few
+// 2^-53); the quotient decides inside it
+__device__ __forceinline__ bool below_rcrit(const OdeConsts& o, double z) {
+  const double t = 3.0 * o.bkoh;
+  if (o.akoh > 0.0) {
+    const double p = z * o.akoh;
+    if (p < t * (1.0 - 1e-12)) return true;
+    if (p > t * (1.0 + 1e-12)) return false;
+  }
+  return z < t / o.akoh;
+}
 // first_unique_criteria (:69-83) given a3 = unique_a3(o.akoh)
 __device__ __forceinline__ bool first_unique_a3(const OdeConsts& o, double rprev, double ziter,
                                                 double a3) {
-  const double akoh = o.akoh;
-  const double bkoh = o.bkoh;
-  const double rcritsqrd = 3.0 * bkoh / akoh;
-  const bool is_ziter_unactivated = ziter < rcritsqrd;
-  const bool is_unactivated = (rprev * rprev < rcritsqrd && is_ziter_unactivated);
-  const double sqrdval = a3 / bkoh;
-  const bool is_subactivated_saturation = (o.s_ratio <= 1.0 + dpow(sqrdval, 0.5));
-  return (is_unactivated && is_subactivated_saturation);
+  const bool is_unactivated = below_rcrit(o, rprev * rprev) && below_rcrit(o, ziter);
+  if (!is_unactivated) return false;
+  const int side = activation_side(o.s_ratio, o.bkoh, a3);
+  return side != 0 ? side < 0 : o.s_ratio <= 1.0 + sqrt(a3 / o.bkoh);
 }
 __device__ __forceinline__ bool first_unique_criteria(const OdeConsts& o, double rprev,
                                                       double ziter) {  // :69-83
@@ -796,43 +1053,34 @@ __device__ __forceinline__ double solve_condensation_fv(const NewtonCfg& c, doub
                                                         double ffactor_fv, double rprev,
                                                         double seed_rsqrd, uint32_t& niters,
                                                         const Where& w) {
-  const OdeConsts o{s_ratio, akoh, bkoh, ffactor_fv};
-  double ziter = initialguess(o, rprev);
+  const OdeConsts o = ode_consts(s_ratio, akoh, bkoh, ffactor_fv);
+  const double z0 = initialguess(o, rprev);
   // ucrit1 || ucrit2: the critical timestep (a general pow) is only needed when ucrit1 fails
-  const bool ucrit1 = first_unique_criteria(o, rprev, ziter);
+  const bool ucrit1 = first_unique_criteria(o, rprev, z0);
   double crit;  // the sub-stepping branch below takes the exact timestep
   const bool direct = ucrit1 || below_critical_timestep(o, delt, crit);
-  double rsqrd;
-  if (direct) {
-    const GEval e0 = eval_g(o, delt, rprev, ziter);
-    // a seed is used when its residual is smaller than the reference guess's; a seeded solve
-    // that does not converge within SEED_MAXITERS, or ends on another root, restarts from the
-    // reference's guess
-    bool done = false;
-    if (seed_ok(seed_rsqrd)) {
-      const GEval es = eval_g(o, delt, rprev, seed_rsqrd);
-      if (fabs(es.g) < fabs(e0.g) && integrate_seeded(c, o, delt, rprev, es, niters, rsqrd) &&
-          seeded_root_ok(o, ucrit1, rsqrd))
-        done = true;
-    }
-    if (!done) rsqrd = integrate_ode(c, o, delt, rprev, e0, niters, w);
-  } else {
-    const double critdelt = critical_timestep(o);
-    const double mindelt = fmax(critdelt, minsubdelt);
-    double remdelt = delt;
-    while (remdelt > 0.0) {
-      if (niters >= NR_ITER_CAP) {
-        w.fail(CLEO_ERR_TIMEOUT);
-        break;
-      }
-      const double subdelt = fmin(mindelt, remdelt);
-      ziter = integrate_ode(c, o, subdelt, rprev, eval_g(o, subdelt, rprev, ziter), niters, w);
-      rprev = dpow(ziter, 0.5);
-      remdelt -= subdelt;
-    }
-    rsqrd = ziter;
+  double z;
+  // a seed is used when its residual is smaller than the reference guess's; a seeded solve that
+  // does not converge within SEED_MAXITERS, or ends on another root, restarts from the
+  // reference's guess
+  bool tried;
+  if (direct && seed_ok(seed_rsqrd) &&
+      integrate_seeded(c, o, delt, rprev, z0, seed_rsqrd, niters, z, tried) &&
+      seeded_root_ok(o, ucrit1, z))
+    return sqrt(z);
+  const double mindelt = direct ? delt : fmax(critical_timestep(o), minsubdelt);
+  bool bad = false;
+  int code = 0;
+  uint32_t n = niters;
+  z = newton_solve<true>(c, o, delt, mindelt, rprev, z0, direct, n, code, bad);
+  if (bad) {
+    n = niters;
+    code = 0;
+    z = newton_solve_wide(c, o, delt, mindelt, rprev, z0, direct, n, code);
   }
-  return sqrt(rsqrd);
+  niters = n;
+  if (code) w.fail(code);
+  return sqrt(z);
 }
 __device__ __forceinline__ double solve_condensation(const NewtonCfg& c, double delt,
                                                      double minsubdelt, double s_ratio,

@@ -949,41 +949,33 @@ k_cs_a(const __grid_constant__ DevCtx c, uint32_t n, const double* __restrict__ 
       const double ffactor = diffusion_factor(press[i], T, psat);
       double akoh, bkoh;
       kohler_factors(msol[i], T, akoh, bkoh);
-      const OdeConsts o{s_ratio[i], akoh, bkoh, ffactor / ventilation_factor(r)};
+      const OdeConsts o = ode_consts(s_ratio[i], akoh, bkoh, ffactor / ventilation_factor(r));
       const double z0 = initialguess(o, r);
       const bool ucrit1 = first_unique_criteria(o, r, z0);
       double crit = 0.0;
       uint32_t ni = 0, carried = 0;
       if (ucrit1 || below_critical_timestep(o, dt, crit)) {
-        bool conv = false, seeded = false, conv1 = false;
-        double z1 = 0.0;
-        GEval e = eval_g(o, dt, r, z0);
+        bool conv = false, seeded = false;
+        double z = 0.0, radius = 0.0, zr = 0.0;
         if (seeds && seed_ok(seeds[i])) {  // the surrogate's seed, when its residual is smaller
-          const GEval es = eval_g(o, dt, r, seeds[i]);
-          if (fabs(es.g) < fabs(e.g)) {
-            double zs;
-            conv = integrate_seeded(cfg, o, dt, r, es, ni, zs) && seeded_root_ok(o, ucrit1, zs);
-            e.z = zs;
-            seeded = true;
+          conv = integrate_seeded(cfg, o, dt, r, z0, seeds[i], ni, z, seeded);
+          if (seeded) {
+            conv = conv && seeded_root_ok(o, ucrit1, z);
+            radius = sqrt(z);
             if (!conv) {
               seeds[i] = -1.0;  // pass B starts from the reference guess
               carried = ni;
             }
           }
         }
-        if (!seeded) {
-          e = nr_iterate(cfg, o, dt, r, e, conv, ni);
-          conv1 = conv;
-          z1 = e.z;
-          e = nr_iterate(cfg, o, dt, r, e, conv, ni);
-        }
+        if (!seeded) conv = two_iterations(cfg, o, dt, r, z0, ni, radius, zr);
         if (conv) {
-          out[i] = max_dryradius(sqrt(e.z), msol[i]);
+          out[i] = max_dryradius(radius, msol[i]);
           if (niters_out) niters_out[i] = ni | (failed ? CLEO_NITERS_FAILED : 0u);
         } else {
           defer = true;  // restart until converged (impliciteuler.cpp:136-140), key 0
           // where pass B's restart continues; NaN after an abandoned seed (a full solve)
-          zres[i] = seeded ? __longlong_as_double(0x7FF8000000000000ll) : (conv1 ? -z1 : e.z);
+          zres[i] = seeded ? __longlong_as_double(0x7FF8000000000000ll) : zr;
         }
       } else {
         defer = true;
@@ -1025,7 +1017,7 @@ k_cs_b(const __grid_constant__ DevCtx c, const double* __restrict__ radius, cons
     if (lkeys[j] == 0u && cfg.maxniters >= 2 && zr == zr) {
       // a direct solve whose two reference iterations in pass A did not converge: the restart
       // continues from them (resume_restart)
-      const OdeConsts o{s_ratio[i], akoh, bkoh, ffactor / ventilation_factor(r)};
+      const OdeConsts o = ode_consts(s_ratio[i], akoh, bkoh, ffactor / ventilation_factor(r));
       ni = 2;
       double rsqrd = 0.0;
       const int code = resume_restart(cfg, o, dt, r, zr, ni, rsqrd);
