@@ -17,7 +17,7 @@
 //                  in their order, their Newton iterations, and the state update
 //   k_b_classify   gridboxes into size buckets (warp-aggregated atomics); the warp kernel's
 //                  buckets as records {gridbox, start, count, RNG slot}
-//   k_b_tv         thread per superdroplet: the pair terminal velocities the warp kernel stages
+//   k_b_perm       thread per gridbox of the warp kernel's buckets: the Fisher-Yates shuffle
 //   k_b_small      persistent, warp per gridbox (n <= small_max <= 128; 64- and 128-slot
 //                  variants): collisions in registers + per-warp shared memory
 //   k_b_cta<false> persistent, CTA per gridbox (small_max < n <= medium_max <= 1024): the same
@@ -355,15 +355,6 @@ k_cond_b(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch 
   }
 }
 
-// ---- the pair terminal velocity of every superdroplet (for the warp kernel), a thread each:
-// the same pair_tv the kernel would evaluate, with every lane busy ----
-__global__ void __launch_bounds__(256) k_b_tv(const __grid_constant__ DevCtx c,
-                                              const __grid_constant__ BatchScratch b) {
-  const uint32_t n = c.counters[0];
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    if (c.sd.gbx[i] < c.ngbxs) b.tv[i] = pair_tv(c.p, c.sd.r[i]);
-}
-
 // ---- size buckets of the gridboxes that hold superdroplets ----
 __global__ void k_b_classify(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b) {
   const uint32_t ng = c.ngbxs;
@@ -456,20 +447,26 @@ __global__ void __launch_bounds__(SEQ_THREADS) k_b_commit_big(const __grid_const
 }
 
 // One pair (2jj, 2jj+1) of the shuffled gridbox, collisions.hpp:140-158, on the drops at indexes
-// a and bb of the staged arrays (tvA, tvB: their pair_tv). The probability and the first random
-// number decide whether the pair's collision happens, which is rare; only then does the
-// out-of-line collide_enact draw the second number (the generator is counter based, so drawing it
-// only then gives the same number) and enact the collision on the staged drops. Pairs that do not
-// collide leave the staged arrays untouched, and the pair loop keeps few registers live.
-static __device__ __noinline__ uint32_t collide_enact(const cleo_b200_params& p,
-                                                      unsigned long long* sx, double* sr,
-                                                      double* sm, uint32_t i1, uint32_t i2,
-                                                      double prob, double phi_coll, uint64_t key,
-                                                      uint64_t slot_out, double tv1, double tv2,
-                                                      const Where& w) {
+// a and bb of the staged arrays. Few pairs collide in a step: a collision needs prob >= 1 or
+// phi_coll < prob (coalescence_gamma's and breakup's own tests), so a pair whose first random
+// number is at least an upper bound of its probability, below 1, is left as it is without
+// evaluating the probability. The bound is single precision (pair_apart); it replaces three FP64
+// divisions, and two correctly rounded powers per pair (Simmel's velocities, a kernel over all
+// superdroplets and 16 bytes of traffic for each before).
+static __device__ __noinline__ uint32_t collide_pair_exact(const cleo_b200_params& p,
+                                                           unsigned long long* sx, double* sr,
+                                                           double* sm, uint32_t a, uint32_t bb,
+                                                           double scale_p, double VOLUME,
+                                                           uint64_t key, uint64_t slot_coll,
+                                                           const Where& w) {
+  const bool swap = sx[a] < sx[bb];  // d1 is the droplet of larger xi
+  const uint32_t i1 = swap ? bb : a, i2 = swap ? a : bb;
   Drop d1{sx[i1], sr[i1], sm[i1]};
   Drop d2{sx[i2], sr[i2], sm[i2]};
-  const double phi_out = cleo_rng_to_unit(cleo_rng_u64(key, slot_out));
+  const double tv1 = pair_tv(p, d1.r), tv2 = pair_tv(p, d2.r);
+  const double prob = scale_p * (double)d1.xi * pair_prob_tv(p, d1.r, d2.r, tv1, tv2, VOLUME);
+  const double phi_coll = cleo_rng_to_unit(cleo_rng_u64(key, slot_coll));
+  const double phi_out = cleo_rng_to_unit(cleo_rng_u64(key, slot_coll + 1));
   // the pair's terminal velocities are the flag's too when both are Simmel's (pair_tv)
   const bool tv_known = p.coll_prob == CLEO_PROB_LONG && p.flag_tv == CLEO_TV_SIMMEL;
   const uint32_t nn = enact_collision(p, d1, d2, prob, phi_coll, phi_out, w, tv_known, tv1, tv2);
@@ -481,32 +478,54 @@ static __device__ __noinline__ uint32_t collide_enact(const cleo_b200_params& p,
   sm[i2] = d2.msol;
   return nn;
 }
-// whether enact_collision changes anything: coalescence (alone or in CoalBuRe) when its gamma
-// (coalescence_gamma, whose min with xi1 / xi2 >= 1 keeps it nonzero) is nonzero, breakup when
-// phi_coll is below the fractional probability
-__device__ __forceinline__ bool collision_happens(const cleo_b200_params& p, double prob,
-                                                  double phi_coll) {
-  if (p.coll_enact == CLEO_ENACT_BREAKUP) return phi_coll < (prob - floor(prob));
-  uint64_t gamma = (uint64_t)floor(prob);
-  if (phi_coll < (prob - (double)gamma)) ++gamma;
-  return gamma != 0;
+// What the probabilities of a gridbox's pairs share, in single precision: scale_p DELT / VOLUME
+// and the kernel's constant, 0.5% up to cover every rounding of the bound.
+__device__ __forceinline__ float pair_bound_coef(const cleo_b200_params& p, uint32_t n,
+                                                 double VOLUME) {
+  const float pairs = (float)(n / 2);
+  float k;
+  if (p.coll_prob == CLEO_PROB_GOLOVIN)
+    k = (float)(1.5e3 * R0 * R0 * R0 * 4.0 / 3.0 * PI);
+  else if (p.coll_prob == CLEO_PROB_LONG)
+    k = (float)(PI * R0 * R0 * W0) * fabsf((float)p.coaleff);
+  else
+    k = fabsf((float)p.const_kernel);
+  return 1.005f * ((float)n * ((float)n - 1.0f)) / (2.0f * pairs) *
+         (k * (float)p.coll_delt / (float)VOLUME);
+}
+// Whether a pair surely does not collide: phi (at most the random number) >= an upper bound of
+// prob. Golovin: r1^3 + r2^3. Long: the collection efficiency (its 1 - k2 / rsmall with 1e-5 to
+// spare), the squared sum of the radii, and for the difference of the terminal velocities the
+// larger droplet's, at most 1.189e-4 r^2 m/s (Simmel's first branch, which the others, 0.06% above
+// it where they meet, stay below beyond) and 9.18. NaN and overflow fail the comparison.
+__device__ __forceinline__ bool pair_apart(const cleo_b200_params& p, float coef, float r1,
+                                           float r2, float xi, float phi) {
+  float k = 1.0f;
+  if (p.coll_prob == CLEO_PROB_LONG) {
+    const float rs = fminf(r1, r2), rb = fmaxf(r1, r2), rb2 = rb * rb, sum = r1 + r2;
+    const float k1 = (float)(4.5e4 * R0 * R0 * 100 * 100), k2 = (float)(3e-4 / R0 / 100);
+    float eff = fmaxf(k1 * rb2 * (1.00001f - __fdividef(k2, rs)), 0.001f);
+    if (!(rb < 49.9f)) eff = fmaxf(eff, 1.0f);
+    k = eff * (sum * sum) * fminf(1.189e-4f / (float)W0 * rb2, 9.18f / (float)W0);
+  } else if (p.coll_prob == CLEO_PROB_GOLOVIN) {
+    k = r1 * r1 * r1 + r2 * r2 * r2;
+  }
+  return phi >= coef * xi * k;
 }
 __device__ __forceinline__ uint32_t collide_pair(const cleo_b200_params& p, unsigned long long* sx,
                                                  double* sr, double* sm, uint32_t a, uint32_t bb,
-                                                 double tvA, double tvB, double scale_p,
-                                                 double VOLUME, uint64_t key, uint64_t slot_pairs,
-                                                 uint32_t jj, const Where& w) {
+                                                 uint32_t n, float coef, double VOLUME,
+                                                 uint64_t key, uint64_t slot_pairs, uint32_t jj,
+                                                 const Where& w) {
   const unsigned long long xa = sx[a], xb = sx[bb];
-  const bool swap = xa < xb;  // d1 is the droplet of larger xi
-  const uint32_t i1 = swap ? bb : a, i2 = swap ? a : bb;
-  const double tv1 = swap ? tvB : tvA, tv2 = swap ? tvA : tvB;
-  const double prob_jk = pair_prob_tv(p, sr[i1], sr[i2], tv1, tv2, VOLUME);
-  const double large_xi = (double)(swap ? xb : xa);
-  const double prob = scale_p * large_xi * prob_jk;
-  const double phi_coll = cleo_rng_to_unit(cleo_rng_u64(key, slot_pairs + 2ull * jj));
-  if (!collision_happens(p, prob, phi_coll)) return 0;
-  return collide_enact(p, sx, sr, sm, i1, i2, prob, phi_coll, key, slot_pairs + 2ull * jj + 1,
-                       tv1, tv2, w);
+  const uint64_t u = cleo_rng_u64(key, slot_pairs + 2ull * jj);
+  // the random number's leading 24 bits, a lower bound of it
+  const float phi = (float)(uint32_t)(u >> 40) * 0x1p-24f;
+  if (pair_apart(p, coef, (float)sr[a], (float)sr[bb], __ull2float_ru(xa < xb ? xb : xa), phi))
+    return 0;
+  const uint32_t npairs = n / 2;
+  const double scale_p = (double)n * ((double)n - 1.0) / (2.0 * (double)npairs);
+  return collide_pair_exact(p, sx, sr, sm, a, bb, scale_p, VOLUME, key, slot_pairs + 2ull * jj, w);
 }
 
 // Fisher-Yates (shuffle.hpp:80-87) applies swap(p[i], p[J[i]]) for i = n-1 down to 1 to the
@@ -539,23 +558,67 @@ using mlp::smem_u32;
 // The 64-slot variant stages all seven 8-byte fields (r, msol, xi, coordinates, id), so its
 // write-back reads shared memory instead of gathering the coordinates and ids from global memory
 // in shuffled order; the 128-slot variant stages r, msol and xi (seven fields of 128 slots would
-// leave room for fewer CTAs per SM than its registers allow). Both stage the pair terminal
-// velocities k_b_tv computed (the last field).
+// leave room for fewer CTAs per SM than its registers allow).
 template <int CAP>
 struct SmallLayout {
   static constexpr bool ALL = CAP <= 64;
-  static constexpr uint32_t NF = ALL ? 8 : 4;  // staged fields per buffer
-  static constexpr uint32_t F_TV = NF - 1;
+  static constexpr uint32_t NF = ALL ? 7 : 3;  // staged fields per buffer
   static constexpr uint32_t BUF = CAP + 2;  // elements per staged field
   static constexpr uint32_t FIELD = BUF * 8;
-  static constexpr uint32_t OFF_P = 2 * NF * FIELD;
-  static constexpr uint32_t OFF_J = OFF_P + CAP;
-  static constexpr uint32_t OFF_F = OFF_J + CAP;  // first index of each swap target (chains)
-  static constexpr uint32_t OFF_BAR = (OFF_F + CAP + 15) / 16 * 16;
+  static constexpr uint32_t OFF_BAR = 2 * NF * FIELD;
   static constexpr uint32_t WARP_BYTES = OFF_BAR + 16;
   static constexpr uint32_t BYTES = WARP_BYTES * B_WARPS;
   static_assert(FIELD % 16 == 0 && WARP_BYTES % 16 == 0, "bulk-copy buffers must be aligned");
 };
+
+// ---- the shuffles of the warp kernel's gridboxes, a thread each ----
+// Fisher-Yates as the reference runs it (shuffle.hpp:80-87): swap(p[i], p[J[i]]) for i = n-1 down
+// to 1, the draws in that order. A thread's permutation is bytes in words of its own bank (word w
+// of lane l at [w][l]), so no two lanes' swaps conflict. Bound by instruction issue, some 60 for a
+// draw and its swap with the lanes of a warp at their own lengths: 15 us for 4.6 M superdroplets,
+// where building and walking the swaps' chains inside the warp kernel, a dependent lookup after
+// another, took about a third of its 170 us. Word w of item it goes to
+// perm[((it / 32) words + w) 32 + it % 32]: written coalesced, and read by the eight consecutive
+// items that a CTA of the warp kernel holds from the same sectors.
+__global__ void __launch_bounds__(B_THREADS)
+k_b_perm(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b, int nq) {
+  __shared__ uint32_t sp[B_WARPS][WARP_MAX / 4][32];
+  const uint32_t t_sdm = *b.tsdm;
+  const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const uint32_t warp = blockIdx.x * B_WARPS + wib, nwarps = gridDim.x * B_WARPS;
+  uint32_t(*W)[32] = sp[wib];
+  uint8_t* B = reinterpret_cast<uint8_t*>(&W[0][lane]);
+  const auto at = [](uint32_t i) { return (i >> 2) * 128 + (i & 3); };
+  for (int q = 0; q < nq; ++q) {
+    const uint32_t count = b.ctr[1 + q];
+    const uint4* list = b.brec + (size_t)q * c.ngbxs;
+    const uint32_t words = (q == 0 ? SMALL_MAX : WARP_MAX) / 4;
+    uint32_t* out = b.perm[q];
+    for (uint32_t it0 = warp * 32; it0 < count; it0 += nwarps * 32) {
+      const uint32_t it = it0 + lane;
+      if (it >= count) continue;
+      const uint4 rec = list[it];
+      const uint32_t n = rec.z, nw = (n + 3) / 4;
+      for (uint32_t w = 0; w < nw; ++w) W[w][lane] = 0x03020100u + 0x04040404u * w;
+      // draw slot + k for i = n-1-k (cleo_rng_u64's counter advanced by one each)
+      uint64_t z = cleo_rng_key(c.p.seed, t_sdm, rec.x) + ((uint64_t)rec.w + 1u) * CLEO_RNG_GOLDEN;
+      for (uint32_t i = n - 1; i > 0; --i) {
+        const uint64_t u = cleo_mix64(z);
+        z += CLEO_RNG_GOLDEN;
+        // cleo_rng_range(u, 0, i + 1) for i + 1 below 2^32
+        const uint64_t m = i + 1;
+        const uint32_t j =
+            (uint32_t)(((u >> 32) * m + (((u & 0xFFFFFFFFull) * m) >> 32)) >> 32);
+        const uint32_t oi = at(i), oj = at(j);
+        const uint8_t t = B[oi];
+        B[oi] = B[oj];
+        B[oj] = t;
+      }
+      uint32_t* o = out + (size_t)(it >> 5) * words * 32 + lane;
+      for (uint32_t w = 0; w < nw; ++w) o[w * 32] = W[w][lane];
+    }
+  }
+}
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
@@ -576,15 +639,13 @@ __global__ void __launch_bounds__(B_THREADS, MINB)
 k_b_small(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b, int q) {
   using L = SmallLayout<CAP>;
   constexpr int H = CAP / 32;
-  static_assert(CAP % 32 == 0 && CAP <= 255, "slot indices are stored as bytes");
+  constexpr uint32_t WORDS = CAP / 4;  // words of a gridbox's permutation (bytes)
+  static_assert(CAP % 32 == 0 && CAP <= 128, "a word of the permutation per lane");
   const uint32_t t_sdm = *b.tsdm;
   extern __shared__ __align__(16) unsigned char smem_small[];
   const cleo_b200_params& p = c.p;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   unsigned char* wsm = smem_small + wib * L::WARP_BYTES;
-  uint8_t* s_p = wsm + L::OFF_P;
-  uint8_t* s_j = wsm + L::OFF_J;
-  uint8_t* s_f = wsm + L::OFF_F;
   uint64_t* bar = reinterpret_cast<uint64_t*>(wsm + L::OFF_BAR);
   const auto field = [&](int buf, int f) { return wsm + (buf * L::NF + f) * L::FIELD; };
   const uint32_t count = b.ctr[1 + q];
@@ -599,7 +660,6 @@ k_b_small(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch
     bulk_g2s(field(buf, 0), c.sd.r + a0, bytes, &bar[buf]);
     bulk_g2s(field(buf, 1), c.sd.msol + a0, bytes, &bar[buf]);
     bulk_g2s(field(buf, 2), c.sd.xi + a0, bytes, &bar[buf]);
-    bulk_g2s(field(buf, L::F_TV), b.tv + a0, bytes, &bar[buf]);
     if constexpr (L::ALL) {
       bulk_g2s(field(buf, 3), c.sd.c3 + a0, bytes, &bar[buf]);
       bulk_g2s(field(buf, 4), c.sd.c1 + a0, bytes, &bar[buf]);
@@ -614,6 +674,12 @@ k_b_small(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch
   const uint4 none = make_uint4(0u, 0u, 0u, 0u);
   uint4 rec_next = item < count ? list[item] : none;
   uint4 rec_after = item + nwarps < count ? list[item + nwarps] : none;
+  // the item's permutation, a word per lane, loaded a gridbox ahead (k_b_perm)
+  const uint32_t* perm = b.perm[q];
+  const auto perm_word = [&](uint32_t it) {
+    return (uint32_t)lane < WORDS ? perm[((size_t)(it >> 5) * WORDS + lane) * 32 + (it & 31)] : 0u;
+  };
+  uint32_t word_next = item < count ? perm_word(item) : 0u;
   uint32_t parity = 0;  // bit k: the phase of bar[k] to wait for
   int cur = 0;
   if (lane == 0) {
@@ -626,6 +692,8 @@ k_b_small(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch
     const uint4 rec = rec_next;
     const uint32_t g = rec.x, base = rec.y, n = rec.z;
     const bool has_next = item + nwarps < count;
+    const uint32_t word = word_next;
+    if (has_next) word_next = perm_word(item + nwarps);
     rec_next = rec_after;
     rec_after = item + 2 * nwarps < count ? list[item + 2 * nwarps] : none;
     // the next gridbox's copies go out before this one's wait
@@ -644,69 +712,25 @@ k_b_small(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch
     double* s_r = reinterpret_cast<double*>(field(cur, 0)) + off;
     double* s_m = reinterpret_cast<double*>(field(cur, 1)) + off;
     unsigned long long* s_x = reinterpret_cast<unsigned long long*>(field(cur, 2)) + off;
-    const double* s_tv = reinterpret_cast<const double*>(field(cur, L::F_TV)) + off;
     const uint64_t key = cleo_rng_key(p.seed, t_sdm, g);
-    const uint64_t slot = rec.w;
-    for (uint32_t k = 1 + lane; k < n; k += 32)
-      s_j[k] = (uint8_t)cleo_rng_range(cleo_rng_u64(key, slot + (n - 1 - k)), 0, (uint64_t)k + 1);
-    __syncwarp();
-    {
-      // origins of the shuffled positions (what fy_origin computes), by chains: tracing position
-      // k through the swaps, nothing happens before swap k, swap k takes it to J[k], and after
-      // that it moves only to a later index s whose J[s] equals its current position. With
-      // FIRST[v] (the first index s >= 1 with J[s] == v) and NEXTSAME[s] (the next index after s
-      // with the same J value), the origin of k is the end of the chain J[k] -> NEXTSAME[k] ->
-      // FIRST[.] -> ... (0 -> FIRST[0] -> ... for k = 0), about ln n lookups instead of n - 1
-      // swaps. Both tables are built from the index groups of 32, last group first, with
-      // __match_any_sync.
-      constexpr uint32_t NONE = 0xFFu;
-      for (uint32_t v = lane; v < n; v += 32) s_f[v] = (uint8_t)NONE;
-      __syncwarp();
-      uint32_t nsame[H];
-#pragma unroll
-      for (int h = H - 1; h >= 0; --h) {
-        nsame[h] = NONE;
-        if (32u * h >= n) continue;  // uniform across the warp
-        const uint32_t sidx = lane + 32u * h;
-        const bool act = sidx >= 1 && sidx < n;
-        const uint32_t v = act ? (uint32_t)s_j[sidx] : 0x100u + lane;  // inactive: unique
-        const unsigned peers = __match_any_sync(0xFFFFFFFFu, v);
-        const unsigned higher = peers & ~((2u << lane) - 1u);
-        if (act) nsame[h] = higher ? 32u * h + __ffs(higher) - 1 : (uint32_t)s_f[v];
-        __syncwarp();
-        if (act && lane == __ffs(peers) - 1) s_f[v] = (uint8_t)sidx;
-        __syncwarp();
-      }
-#pragma unroll
-      for (int h = 0; h < H; ++h) {
-        const uint32_t k = lane + 32u * h;
-        if (k < n) {
-          uint32_t cur = k == 0 ? 0u : (uint32_t)s_j[k];
-          uint32_t nx = k == 0 ? (uint32_t)s_f[0] : nsame[h];
-          while (nx != NONE) {  // strictly increasing, so at most n hops
-            cur = nx;
-            nx = s_f[cur];
-          }
-          s_p[k] = (uint8_t)cur;
-        }
-      }
-    }
-    __syncwarp();
-    const uint64_t slot_pairs = slot + (n >= 1 ? n - 1 : 0);
+    const uint64_t slot_pairs = (uint64_t)rec.w + (n - 1);
     const uint32_t npairs = n / 2;
-    const double scale_p = (double)n * ((double)n - 1.0) / (2.0 * (double)npairs);
+    const float coef = pair_bound_coef(p, n, VOLUME);
     uint32_t nnull = 0;
-    for (uint32_t jj = lane; jj < npairs; jj += 32) {
-      const uint32_t a = s_p[2 * jj], bb = s_p[2 * jj + 1];
-      const Where w{c.err, g, (uint64_t)base + 2 * jj};
-      nnull += collide_pair(p, s_x, s_r, s_m, a, bb, s_tv[a], s_tv[bb], scale_p, VOLUME, key,
-                            slot_pairs, jj, w);
+    for (uint32_t j0 = 0; j0 < npairs; j0 += 32) {  // positions 2jj, 2jj + 1: word jj / 2
+      const uint32_t jj = j0 + lane;
+      const uint32_t pw = __shfl_sync(0xFFFFFFFFu, word, (jj >> 1) & 31) >> (16 * (jj & 1));
+      if (jj < npairs) {
+        const uint32_t a = pw & 0xFFu, bb = (pw >> 8) & 0xFFu;
+        const Where w{c.err, g, (uint64_t)base + 2 * jj};
+        nnull += collide_pair(p, s_x, s_r, s_m, a, bb, n, coef, VOLUME, key, slot_pairs, jj, w);
+      }
     }
     __syncwarp();
     const uint32_t totnull = warp_sum_u(nnull);
     const uint32_t nvalid = n - totnull;
     // destinations: valid superdroplets in shuffled order, then the nulls (collisions.hpp:240-248)
-    uint32_t src[H], q[H];
+    uint32_t src[H], dst[H];
     double c3v[L::ALL ? 1 : H], c1v[L::ALL ? 1 : H], c2v[L::ALL ? 1 : H];
     unsigned long long idv[L::ALL ? 1 : H];
     uint32_t cval = 0, cnull = 0;
@@ -715,12 +739,13 @@ k_b_small(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch
       if (32u * h >= n) break;  // uniform across the warp
       const uint32_t k = lane + 32 * h;
       const bool act = k < n;
-      src[h] = act ? s_p[k] : 0;
+      const uint32_t pw = __shfl_sync(0xFFFFFFFFu, word, (k >> 2) & 31);
+      src[h] = act ? (pw >> (8 * (k & 3))) & 0xFFu : 0;
       const bool valid = act && s_x[src[h]] != 0;
       const unsigned mv = __ballot_sync(0xFFFFFFFFu, valid);
       const unsigned mn = __ballot_sync(0xFFFFFFFFu, act && !valid);
       const unsigned lt = (1u << lane) - 1u;
-      q[h] = valid ? cval + __popc(mv & lt) : nvalid + cnull + __popc(mn & lt);
+      dst[h] = valid ? cval + __popc(mv & lt) : nvalid + cnull + __popc(mn & lt);
       cval += __popc(mv);
       cnull += __popc(mn);
       if constexpr (!L::ALL) {
@@ -738,11 +763,11 @@ k_b_small(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch
     for (int h = 0; h < H; ++h) {
       const uint32_t k = lane + 32 * h;
       if (k < n) {
-        const uint32_t o = base + q[h];
+        const uint32_t o = base + dst[h];
         c.sd.r[o] = s_r[src[h]];
         c.sd.msol[o] = s_m[src[h]];
         c.sd.xi[o] = s_x[src[h]];
-        c.sd.gbx[o] = q[h] < nvalid ? g : OOB;
+        if (dst[h] >= nvalid) c.sd.gbx[o] = OOB;  // the range's indexes are g already
         if constexpr (L::ALL) {
           c.sd.c3[o] = reinterpret_cast<const double*>(field(cur, 3))[off + src[h]];
           c.sd.c1[o] = reinterpret_cast<const double*>(field(cur, 4))[off + src[h]];
@@ -867,9 +892,6 @@ k_b_cta(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b
     uint32_t* P = LARGE ? c.scr_p + base : reinterpret_cast<uint32_t*>(smem + 24 * MBUF);
     uint32_t* J = LARGE ? c.scr_j + base
                         : reinterpret_cast<uint32_t*>(smem + 24 * MBUF + 4 * MEDIUM_MAX);
-    // the pair terminal velocities k_b_tv computed (medium: copied to shared memory after the five
-    // staged arrays; large: read per pair)
-    double* Stv = LARGE ? nullptr : reinterpret_cast<double*>(smem + 24 * MBUF + 8 * MEDIUM_MAX);
     if (!LARGE) {
       if (tid == 0) {  // the previous gridbox's accesses ended at the barriers above
         const uint32_t bytes = ((n + off + 1u) & ~1u) * 8u;
@@ -894,8 +916,6 @@ k_b_cta(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b
         Sr[k] = c.sd.r[base + k];
         Sm[k] = c.sd.msol[base + k];
         Sx[k] = c.sd.xi[base + k];
-      } else {
-        Stv[k] = b.tv[base + k];  // k_b_tv's pair terminal velocity of the same radius
       }
       if (k >= 1) J[k] = (uint32_t)cleo_rng_range(cleo_rng_u64(key, slot + (n - 1 - k)), 0, (uint64_t)k + 1);
     }
@@ -921,16 +941,13 @@ k_b_cta(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b
     __syncthreads();
     const uint64_t slot_pairs = slot + (n >= 1 ? n - 1 : 0);
     const uint32_t npairs = n / 2;
-    const double scale_p = (double)n * ((double)n - 1.0) / (2.0 * (double)npairs);
     const double VOLUME = c.volume[g] * VOL0;
+    const float coef = pair_bound_coef(p, n, VOLUME);
     uint32_t nnull = 0;
     for (uint32_t jj = tid; jj < npairs; jj += NT) {
       const uint32_t a = P[2 * jj], bb = P[2 * jj + 1];
       const Where w{c.err, g, (uint64_t)base + 2 * jj};
-      const double tvA = LARGE ? b.tv[base + a] : Stv[a];
-      const double tvB = LARGE ? b.tv[base + bb] : Stv[bb];
-      nnull += collide_pair(p, Sx, Sr, Sm, a, bb, tvA, tvB, scale_p, VOLUME, key, slot_pairs, jj,
-                            w);
+      nnull += collide_pair(p, Sx, Sr, Sm, a, bb, n, coef, VOLUME, key, slot_pairs, jj, w);
     }
     const uint32_t totnull = block_sum(nnull, shw);
     const uint32_t nvalid = n - totnull;
@@ -964,7 +981,7 @@ k_b_cta(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b
         c.sd.r[o] = Sr[src];
         c.sd.msol[o] = Sm[src];
         c.sd.xi[o] = Sx[src];
-        c.sd.gbx[o] = q < nvalid ? g : OOB;
+        if (q >= nvalid) c.sd.gbx[o] = OOB;
         c.sd.c3[o] = c.scr_c3[o];
         c.sd.c1[o] = c.scr_c1[o];
         c.sd.c2[o] = c.scr_c2[o];
@@ -994,7 +1011,7 @@ k_b_cta(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b
           c.sd.r[o] = Sr[src];
           c.sd.msol[o] = Sm[src];
           c.sd.xi[o] = Sx[src];
-          c.sd.gbx[o] = q < nvalid ? g : OOB;
+          if (q >= nvalid) c.sd.gbx[o] = OOB;
           c.sd.c3[o] = c3v[h];
           c.sd.c1[o] = c1v[h];
           c.sd.c2[o] = c2v[h];

@@ -5,12 +5,11 @@
 
 namespace {
 
-constexpr uint32_t SMALL_MAX = 64;   // default limit of the warp kernel
-constexpr uint32_t WARP_MAX = 128;   // largest gridbox the warp kernel's 128-slot variant holds
+constexpr uint32_t SMALL_MAX = 64;   // largest gridbox of the warp kernel's 64-slot variant
+constexpr uint32_t WARP_MAX = 128;   // and of its 128-slot variant (the default limit)
 constexpr uint32_t MEDIUM_MAX = 1024;
-// r, msol, xi (each with two elements of slack for the bulk copies' alignment), P, J, Simmel
-// velocity
-constexpr uint32_t MEDIUM_SMEM = 24 * (MEDIUM_MAX + 2) + 16 * MEDIUM_MAX;
+// r, msol, xi (each with two elements of slack for the bulk copies' alignment), P, J
+constexpr uint32_t MEDIUM_SMEM = 24 * (MEDIUM_MAX + 2) + 8 * MEDIUM_MAX;
 constexpr uint32_t FY_PARALLEL_MAX = 256;  // gridboxes up to this size shuffle in parallel
 constexpr int B_THREADS = 256;
 constexpr int B_WARPS = B_THREADS / 32;
@@ -25,14 +24,13 @@ struct BatchScratch {
   uint32_t* its;     // per superdroplet Newton iterations
   double* qm;        // per superdroplet condensate mass x xi before the solves, when the first
                      // condensation sub-step after motion also gives qcond (else null)
-  double* tv;        // per superdroplet pair terminal velocity (pair_tv) for the warp kernel,
-                     // two elements of padding for its bulk copies
   double* zres;      // per deferred direct solve: pass A's iterate that pass B resumes from
   double* ffv;       // per deferred solve: pass A's diffusion factor over the ventilation factor
   uint32_t* lkeys;   // cost keys of deferred solves
   uint32_t* lvals;   // positions of deferred solves
   uint32_t* bucket;  // [4][ngbxs] gridbox lists per size bucket
   uint4* brec;       // [2][ngbxs] the warp kernel's buckets as {gridbox, start, count, RNG slot}
+  uint32_t* perm[2];  // the shuffles of those buckets' gridboxes (k_b_perm): 16 and 32 words each
   uint32_t* slot;    // per gridbox RNG slot offset within the SDM step
   uint32_t* ctr;     // [0] deferred solves, [1..4] bucket counts, [5..8] bucket heads,
                      // [9] restarts among the deferred solves, [10] big gridboxes (commit)

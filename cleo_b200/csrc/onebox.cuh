@@ -220,8 +220,8 @@ __global__ void k_ob_pairs(const __grid_constant__ DevCtx c, const __grid_consta
   const uint32_t* first = o.first;
   const uint64_t key = cleo_rng_key(c.p.seed, *b.tsdm, 0);
   const uint64_t slot_pairs = (uint64_t)b.slot[0] + (n >= 1 ? n - 1 : 0);
-  const double scale_p = (double)n * ((double)n - 1.0) / (2.0 * (double)npairs);
   const double VOLUME = c.volume[0] * VOL0;
+  const float coef = pair_bound_coef(c.p, n, VOLUME);
   uint32_t nnull = 0, ninv = 0;
   for (uint32_t jj = blockIdx.x * blockDim.x + threadIdx.x; jj <= npairs;
        jj += gridDim.x * blockDim.x) {
@@ -237,9 +237,8 @@ __global__ void k_ob_pairs(const __grid_constant__ DevCtx c, const __grid_consta
         o.P[2 * jj + 1] = bb;
       }
       const Where w{c.err, 0u, (uint64_t)base + 2 * jj};
-      nnull += collide_pair(c.p, c.sd.xi + base, c.sd.r + base, c.sd.msol + base, a, bb,
-                            b.tv[base + a], b.tv[base + bb], scale_p, VOLUME, key, slot_pairs,
-                            jj, w);
+      nnull += collide_pair(c.p, c.sd.xi + base, c.sd.r + base, c.sd.msol + base, a, bb, n, coef,
+                            VOLUME, key, slot_pairs, jj, w);
       const uint32_t fa = c.sd.xi[base + a] != 0 ? 1u : 0u;
       const uint32_t fb = c.sd.xi[base + bb] != 0 ? 1u : 0u;
       o.vflag[2 * jj] = fa;

@@ -190,7 +190,9 @@ struct cleo_b200_ctx {
     int small_minb;       // 64-slot warp kernel: resident CTAs per SM it is compiled for
     int condb_minb;       // pass-B variant (3, 4 or 5), tuned apart from pass A's
   };
-  TuneCfg cfg{256, 3, SMALL_MAX, 2, 3};
+  // (gridboxes of 65 .. 128 superdroplets to the warp kernel's 128-slot variant: on the uneven 3-D
+  // workload a CTA each takes 348 us for what it does in 46)
+  TuneCfg cfg{256, 4, WARP_MAX, 2, 3};
   std::vector<TuneCfg> cand;
   std::vector<double> t_cond, t_condb, t_coll;
   size_t tune_step = 0, tune_total = 0;
@@ -1249,6 +1251,7 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
     x->launches += 1;
   }
   uint32_t subt = t_sdm;
+  int colls = 0;  // collision sub-steps so far
   while (subt < t_sdm_next) {
     const bool cond = on_step(d.p.condstep, subt);
     const bool coll = on_step(d.p.collstep, subt);
@@ -1303,10 +1306,6 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
       StageMark mk(x, 4);
       const OneBox& o = x->ob;
       const int go = grid_for((size_t)d.slots + 1, 256);
-      if (d.p.coll_prob == CLEO_PROB_LONG) {  // otherwise the pair terminal velocities stay 0
-        k_b_tv<<<grid_for(d.slots, 256), 256, 0, s>>>(d, b);
-        x->launches += 1;
-      }
       // scans of n + 1 entries (entries past n unused): one block while the slots allow
       const bool one_block = (uint64_t)d.slots + 1 <= OB_SCAN_MAX;
       const auto scan = [&](uint32_t* a, const uint32_t* skip) {
@@ -1337,16 +1336,17 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
       x->launches += 2;
     } else if (coll) {
       StageMark mk(x, 4);
-      k_b_reset<<<1, 32, 0, s>>>(d, b, 0);
-      k_b_classify<<<gg, 256, 0, s>>>(d, b);
-      if (d.p.coll_prob == CLEO_PROB_LONG) {  // otherwise the pair terminal velocities stay 0
-        k_b_tv<<<grid_for(d.slots, 256), 256, 0, s>>>(d, b);
+      if (colls++ > 0) {  // (the step's first finds its counters reset by k_b_reset above)
+        k_b_reset<<<1, 32, 0, s>>>(d, b, 0);
         x->launches += 1;
       }
+      k_b_classify<<<gg, 256, 0, s>>>(d, b);
       // the warp kernel's 64-slot variant takes gridboxes up to 64 superdroplets, its 128-slot
       // variant those of 65 .. small_max (when small_max > 64)
       const int wide = x->cfg.small_max > SMALL_MAX ? 1 : 0, m3 = x->cfg.small_minb == 3 ? 1 : 0;
       constexpr uint32_t SW = SmallLayout<WARP_MAX>::BYTES, SS = SmallLayout<SMALL_MAX>::BYTES;
+      k_b_perm<<<grid_for(((size_t)d.ngbxs + 31) / 32 * 32, B_THREADS), B_THREADS, 0, s>>>(
+          d, b, 1 + wide);
       if (m3)
         k_b_small<3, SMALL_MAX><<<x->grid_small[1], B_THREADS, SS, s>>>(d, b, 0);
       else
@@ -1641,7 +1641,6 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   rc |= dalloc(x, &x->bs.th_u3, ng);
   rc |= dalloc(x, &x->bs.dm, cap);
   rc |= dalloc(x, &x->bs.its, cap);
-  rc |= dalloc(x, &x->bs.tv, cap + 2);
   rc |= dalloc(x, &x->qm_buf, cap);
   if (ng == 1) {  // one gridbox: its collisions by the whole GPU (onebox.cuh)
     OneBox& o = x->ob;
@@ -1660,6 +1659,8 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   rc |= dalloc(x, &x->bs.bucket, 4 * ng);
   rc |= dalloc(x, &x->bs.big, ng);
   rc |= dalloc(x, &x->bs.brec, 2 * ng);
+  for (int q = 0; q < 2; ++q)  // whole blocks of 32 gridboxes
+    rc |= dalloc(x, &x->bs.perm[q], (ng + 31) / 32 * 32 * ((q == 0 ? SMALL_MAX : WARP_MAX) / 4));
   rc |= dalloc(x, &x->bs.slot, ng);
   rc |= dalloc(x, &x->bs.ctr, 12);
   rc |= dalloc(x, &x->bs.tsdm, 1);
@@ -1730,8 +1731,6 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   CUDA_TRY(cudaMemsetAsync(d.pg_flag, 0, (size_t)d.npages * 4, x->stream));
   CUDA_TRY(cudaMemsetAsync(d.pg_ctr, 0, 16, x->stream));
   CUDA_TRY(cudaMemsetAsync(d.mv_stamp, 0, (size_t)d.ngbxs * 4, x->stream));
-  // pair terminal velocities: 0 unless the Long kernel's k_b_tv writes them
-  CUDA_TRY(cudaMemsetAsync(x->bs.tv, 0, ((size_t)d.slots + 2) * 8, x->stream));
   if (x->one_box) {  // the one-box counts start at zero (k_ob_gather clears what a step used)
     CUDA_TRY(cudaMemsetAsync(x->ob.cnt, 0, ((size_t)d.slots + 2) * 4, x->stream));
     CUDA_TRY(cudaMemsetAsync(x->ob.fill, 0, ((size_t)d.slots + 2) * 4, x->stream));
