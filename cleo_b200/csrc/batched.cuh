@@ -8,7 +8,7 @@
 //   k_cond_a       thread per superdroplet: the mandatory two Newton iterations of every
 //                  implicit-Euler solve; solves needing more (sub-stepping, or a restart after two
 //                  unconverged iterations) are appended to a list keyed by their cost
-//   (radix sort of that list by cost, 16-bit keys)
+//   k_cond_place   that list by cost class
 //   k_mlp_tc       with nr_seed = CLEO_NRSEED_MLP only: the surrogate's Newton seeds for the
 //                  listed solves (the ones the reference guess did not settle in two iterations)
 //   k_cond_b       thread per listed solve, neighbouring lanes of similar cost, from the seed
@@ -32,6 +32,12 @@
 #pragma once
 
 namespace {
+
+using mlp::fence_async_smem;
+using mlp::mbar_init;
+using mlp::mbar_wait_bounded;
+using mlp::MBAR_TRIES;
+using mlp::smem_u32;
 
 __device__ __forceinline__ uint32_t warp_sum_u(uint32_t v) {
 #pragma unroll
@@ -199,9 +205,15 @@ __global__ void __launch_bounds__(SEQ_THREADS) k_b_qcond(const __grid_constant__
 // ---- per-gridbox thermodynamics of superdroplets_change (condensation.cpp:43-59) ----
 // (every gridbox, empty ones too: the reference evaluates psat for each, and its check of the
 // temperature with it)
-__global__ void k_b_thermo(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b) {
+// With `first` (an SDM step that begins with condensation) it also does k_b_reset's part.
+__global__ void k_b_thermo(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b,
+                           int first) {
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+  if (tid < 2 * COST_CLASSES) b.ccnt[tid] = 0;
+  if (first && tid < 8) b.ctr[1 + tid] = 0;  // bucket counts and heads
   for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < c.ngbxs; g += gridDim.x * blockDim.x) {
-    if (g == 0) b.ctr[0] = b.ctr[9] = b.ctr[10] = 0;  // deferred solves, restarts, big gridboxes
+    if (g == 0) b.ctr[0] = b.ctr[10] = 0;  // deferred solves, big gridboxes
+    if (first) b.slot[g] = 0;
     const Where w{c.err, g, c.gstart[g]};
     const double temp = c.temp[g];
     const double psat = saturation_pressure(temp, w);
@@ -214,8 +226,8 @@ __global__ void k_b_thermo(const __grid_constant__ DevCtx c, const __grid_consta
   }
 }
 
-// the surrogate's IO for the batched schedule: row j is the j-th solve of pass A's sorted list,
-// whose first b.ctr[9] entries are the direct solves that two iterations did not settle (key 0;
+// the surrogate's IO for the batched schedule: row j is the j-th of pass A's solves by class,
+// whose first b.ccnt[0] entries are the direct solves that two iterations did not settle (key 0;
 // the sub-stepping solves after them cannot use a seed); the seed r^2 goes to b.dm of that
 // droplet, which pass B reads (and then overwrites with the droplet's condensed mass)
 struct SdmListSeedIO {
@@ -240,68 +252,142 @@ struct SdmListSeedIO {
   }
 };
 
-// cost key of a deferred solve: number of sub-steps (0 for a restart of the unique branch)
-__device__ __forceinline__ uint32_t deferred_key(double delt, double mindelt, bool substep) {
-  if (!substep) return 0u;
+// cost class of a deferred solve of `delt / mindelt` sub-steps: 1 + a quarter-octave of their number,
+// read off the leading bits of the single-precision value; class 0 is the restarts of direct solves
+__device__ __forceinline__ uint32_t cost_class(double delt, double mindelt) {
   const double ns = ceil(delt / mindelt);
-  return ns >= 65535.0 ? 65535u : (uint32_t)ns;
+  const float f = ns >= 1.0 ? (ns <= 65535.0 ? (float)ns : 65536.0f) : 1.0f;
+  return 1u + ((__float_as_uint(f) >> 21) - (127u << 2));  // 1 .. 65
+}
+// the appended solves counted per class, a block's in shared memory first; every thread of the block
+// calls these. The restarts, most of the solves at a tight tolerance, are counted a warp at a time in
+// a register (one shared atomic each ran 32 in a row: 50 us of 275 for 5 M superdroplets).
+__device__ __forceinline__ void class_count_begin(uint32_t* cnt) {
+  for (uint32_t i = threadIdx.x; i < COST_CLASSES; i += blockDim.x) cnt[i] = 0;
+  __syncthreads();
+}
+__device__ __forceinline__ void class_count(uint32_t* cnt, uint32_t& restarts, bool defer,
+                                            uint32_t cls) {
+  restarts += __popc(__ballot_sync(0xFFFFFFFFu, defer && cls == 0u));
+  if (defer && cls != 0u) atomicAdd(&cnt[cls], 1u);
+}
+__device__ __forceinline__ void class_count_end(uint32_t* cnt, uint32_t restarts,
+                                                uint32_t* total) {
+  if ((threadIdx.x & 31) == 0 && restarts) atomicAdd(&cnt[0], restarts);
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < COST_CLASSES; i += blockDim.x)
+    if (cnt[i]) atomicAdd(&total[i], cnt[i]);
+}
+// The deferred solves by class, restarts first. Only neighbouring lanes' costs matter to pass B
+// (and the restarts' place to the surrogate), not the order within a class, so blocks of
+// PLACE_ITEMS solves take their shares of each class with one atomic: one launch where a radix
+// sort of the 16-bit costs took eleven, which returned at once or not (about 16 us of a step), and
+// 7 us where it sorted 400 thousand in 30.
+constexpr uint32_t PLACE_ITEMS = 1024;
+__global__ void __launch_bounds__(256)
+k_cond_place(const uint32_t* __restrict__ n_ptr, const uint32_t* __restrict__ lkeys,
+             const uint32_t* __restrict__ lvals, uint32_t* __restrict__ ccnt,
+             uint32_t* __restrict__ order) {
+  __shared__ uint32_t cnt[COST_CLASSES], start[COST_CLASSES], total[COST_CLASSES];
+  const uint32_t nl = *n_ptr;
+  constexpr uint32_t PER = PLACE_ITEMS / 256;
+  if (threadIdx.x < COST_CLASSES) total[threadIdx.x] = ccnt[threadIdx.x];
+  for (uint32_t i0 = blockIdx.x * PLACE_ITEMS; i0 < nl; i0 += gridDim.x * PLACE_ITEMS) {
+    class_count_begin(cnt);
+    uint32_t cls[PER], val[PER], rank[PER];
+#pragma unroll
+    for (uint32_t q = 0; q < PER; ++q) {
+      const uint32_t i = i0 + q * 256 + threadIdx.x;
+      cls[q] = i < nl ? lkeys[i] : COST_CLASSES;
+      val[q] = i < nl ? lvals[i] : 0u;
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < PER; ++q) {  // one shared atomic per class a warp meets
+      const unsigned peers = __match_any_sync(0xFFFFFFFFu, cls[q]);
+      const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+      uint32_t base = 0;
+      if (lane == leader && cls[q] < COST_CLASSES)
+        base = atomicAdd(&cnt[cls[q]], (uint32_t)__popc(peers));
+      rank[q] = __shfl_sync(0xFFFFFFFFu, base, leader) + __popc(peers & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    if (threadIdx.x < COST_CLASSES) {
+      const uint32_t m = cnt[threadIdx.x];
+      uint32_t s = m ? atomicAdd(&ccnt[COST_CLASSES + threadIdx.x], m) : 0u;
+      for (uint32_t k = 0; k < threadIdx.x; ++k) s += total[k];
+      start[threadIdx.x] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t q = 0; q < PER; ++q)
+      if (cls[q] < COST_CLASSES) order[start[cls[q]] + rank[q]] = val[q];
+    __syncthreads();
+  }
 }
 
 // ---- pass A: superdrop_mass_change (condensation.cpp:98-112) up to two Newton iterations ----
+// Bound by issue (930 instructions a warp of droplets, 400 of them FP64) and by the loads at the head
+// of each solve. A resident grid walks the slots, so the blocks' class counts are few; the gridbox
+// index, behind which the gridbox's values wait, is loaded a slot ahead. (Copying the next slot's
+// eight values ahead into shared memory as well was slower, 281 us for 225 on 5 M superdroplets: a
+// warp's copies of one gridbox's value are 32 separate ones.)
 template <int MINB>
 __global__ void __launch_bounds__(256, MINB)
 k_cond_a(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b) {
   const cleo_b200_params& p = c.p;
   const uint32_t n = c.counters[0];
   const NewtonCfg cfg{p.maxniters, p.rtol, p.atol};
-  for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
-    const uint32_t i = i0 + threadIdx.x;
+  __shared__ uint32_t cnt[COST_CLASSES];
+  class_count_begin(cnt);
+  uint32_t restarts = 0;
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x;
+  uint32_t g_next = i0 + threadIdx.x < n ? c.sd.gbx[i0 + threadIdx.x] : OOB;
+  for (; i0 < n; i0 += step) {
+    const uint32_t i = (uint32_t)i0 + threadIdx.x;
+    const uint32_t g = g_next;
+    g_next = i0 + step + threadIdx.x < n ? c.sd.gbx[i0 + step + threadIdx.x] : OOB;
     bool defer = false;
     uint32_t key = 0;
-    if (i < n) {
-      const uint32_t g = c.sd.gbx[i];
-      if (g < c.ngbxs) {
-        const Where w{c.err, g, i};
-        const double r = c.sd.r[i], msol = c.sd.msol[i];
-        // the condensate mass qcond sums (k_b_qcond's term), for the commit to add in order
-        if (b.qm) b.qm[i] = condensate_mass(r, msol, w) * (double)c.sd.xi[i];
-        const double ffactor_fv = b.th_ff[g] / ventilation_factor(r);
-        const OdeConsts o = ode_consts(b.th_s[g], b.th_ak[g], kohler_b(msol), ffactor_fv);
-        const double z0 = initialguess_a3(o, r, b.th_a3[g]);
-        // ucrit1 || ucrit2, the critical timestep only evaluated when ucrit1 fails
-        const bool ucrit1 = first_unique_a3(o, r, z0, b.th_u3[g]);
-        double crit = 0.0;
-        uint32_t ni = 0;
-        if (ucrit1 || below_critical_timestep(o, p.cond_delt, crit)) {
-          double radius, zres;
-          if (!two_iterations(cfg, o, p.cond_delt, r, z0, ni, radius, zres)) {
-            defer = true;  // restart from z0 until converged (impliciteuler.cpp:136-140)
-            b.zres[i] = zres;
-            b.ffv[i] = ffactor_fv;
-          } else {
-            const double rnew = max_dryradius(radius, msol);  // change_radius
-            b.dm[i] = (condensate_mass(rnew, msol, w) - condensate_mass(r, msol, w)) *
-                      (double)c.sd.xi[i];
-            b.its[i] = ni;
-            c.sd.r[i] = rnew;
-          }
+    if (g < c.ngbxs) {
+      const Where w{c.err, g, i};
+      const double r = c.sd.r[i], msol = c.sd.msol[i];
+      // the condensate mass qcond sums (k_b_qcond's term), for the commit to add in order
+      if (b.qm) b.qm[i] = condensate_mass(r, msol, w) * (double)c.sd.xi[i];
+      const double ffactor_fv = b.th_ff[g] / ventilation_factor(r);
+      const OdeConsts o = ode_consts(b.th_s[g], b.th_ak[g], kohler_b(msol), ffactor_fv);
+      const double z0 = initialguess_a3(o, r, b.th_a3[g]);
+      // ucrit1 || ucrit2, the critical timestep only evaluated when ucrit1 fails
+      const bool ucrit1 = first_unique_a3(o, r, z0, b.th_u3[g]);
+      double crit = 0.0;
+      uint32_t ni = 0;
+      if (ucrit1 || below_critical_timestep(o, p.cond_delt, crit)) {
+        double radius, zres;
+        if (!two_iterations(cfg, o, p.cond_delt, r, z0, ni, radius, zres)) {
+          defer = true;  // restart from z0 until converged (impliciteuler.cpp:136-140)
+          b.zres[i] = zres;
+          b.ffv[i] = ffactor_fv;
         } else {
-          defer = true;
-          key = deferred_key(p.cond_delt, fmax(crit, p.cond_minsubdelt), true);
-          b.ffv[i] = ffactor_fv;  // pass B's sub-stepping solve starts from it
+          const double rnew = max_dryradius(radius, msol);  // change_radius
+          b.dm[i] = (condensate_mass(rnew, msol, w) - condensate_mass(r, msol, w)) *
+                    (double)c.sd.xi[i];
+          b.its[i] = ni;
+          c.sd.r[i] = rnew;
         }
+      } else {
+        defer = true;
+        key = cost_class(p.cond_delt, fmax(crit, p.cond_minsubdelt));
+        b.ffv[i] = ffactor_fv;  // pass B's sub-stepping solve starts from it
       }
     }
     const uint32_t pos = warp_append(&b.ctr[0], defer);
-    {  // restarts (key 0) lead the sorted list; their number bounds the surrogate's rows
-      const unsigned rm = __ballot_sync(0xFFFFFFFFu, defer && key == 0u);
-      if (rm && (threadIdx.x & 31) == (unsigned)(__ffs(rm) - 1)) atomicAdd(&b.ctr[9], __popc(rm));
-    }
     if (defer) {
       b.lkeys[pos] = key;
       b.lvals[pos] = i;
     }
+    class_count(cnt, restarts, defer, key);
   }
+  class_count_end(cnt, restarts, b.ccnt);
 }
 
 // ---- pass B: the deferred solves, in order of cost ----
@@ -309,14 +395,14 @@ template <int MINB>
 __global__ void __launch_bounds__(256, MINB)
 k_cond_b(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b) {
   const cleo_b200_params& p = c.p;
-  const uint32_t nl = b.ctr[0];
+  const uint32_t nl = b.ctr[0], restarts = b.ccnt[0];
   const NewtonCfg cfg{p.maxniters, p.rtol, p.atol};
   for (uint32_t jr = blockIdx.x * blockDim.x + threadIdx.x; jr < nl;
        jr += gridDim.x * blockDim.x) {
     // the list is sorted by ascending cost: the most expensive solves start first, so that the
     // longest sub-stepping ones do not run alone at the end
     const uint32_t j = nl - 1 - jr;
-    const uint32_t i = b.lvals[j];
+    const uint32_t i = b.order[j];
     const uint32_t g = c.sd.gbx[i];
     const Where w{c.err, g, i};
     const double r = c.sd.r[i], msol = c.sd.msol[i];
@@ -324,7 +410,7 @@ k_cond_b(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch 
     uint32_t ni = 0;
     const double seed = p.nr_seed == CLEO_NRSEED_MLP ? b.dm[i] : 0.0;
     double newr;
-    if (b.lkeys[j] == 0u && cfg.maxniters >= 2) {
+    if (j < restarts && cfg.maxniters >= 2) {
       // a direct solve whose two iterations in pass A did not converge: the restart continues
       // from them (resume_restart), unless the surrogate's seed converges first
       const OdeConsts o = ode_consts(b.th_s[g], akoh, bkoh, b.ffv[i]);  // pass A's th_ff / ventilation
@@ -549,11 +635,6 @@ __device__ __forceinline__ uint32_t fy_origin(const JT* J, uint32_t n, uint32_t 
 // in flight while the current one is processed. A copy starts at the even element at or below
 // the gridbox's first superdroplet (16-byte alignment) and covers an even number of elements, so
 // it may read one element past the range (the SoA arrays carry two elements of padding).
-using mlp::fence_async_smem;
-using mlp::mbar_init;
-using mlp::mbar_wait_bounded;
-using mlp::MBAR_TRIES;
-using mlp::smem_u32;
 
 // The 64-slot variant stages all seven 8-byte fields (r, msol, xi, coordinates, id), so its
 // write-back reads shared memory instead of gathering the coordinates and ids from global memory

@@ -88,109 +88,90 @@ __global__ void k_keys_paged(const __grid_constant__ DevCtx c, uint32_t* __restr
     vals[i] = i;
   }
 }
-// gp[k] = first sorted position with key >= k, k = 0 .. ngbxs + 1 (findrefs.hpp:54-126)
+// gp[k] = first sorted position with key >= k, k = 0 .. ngbxs + 1 (findrefs.hpp:54-126). Every page
+// holds its superdroplets and PAGE_SLACK free slots, so the page starts follow from gp alone. The
+// out-of-domain store's old count goes to counters[3], where k_gather_paged appends.
 __global__ void k_lower_bounds(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ keys,
                                uint32_t* __restrict__ gp) {
   const uint32_t n = c.counters[0];
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < c.ngbxs + 2;
-       k += gridDim.x * blockDim.x)
-    gp[k] = lower_bound_u32(keys, n, k);
-}
-// slots of each page: its superdroplets plus the slack (scanned into pstart)
-__global__ void k_pg_sizes_full(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ gp,
-                                uint32_t* __restrict__ psize) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < c.npages;
-       p += gridDim.x * blockDim.x) {
-    const uint32_t lo = p * PAGE_GBXS, hi = min(lo + PAGE_GBXS, c.ngbxs);
-    psize[p] = gp[hi] - gp[lo] + PAGE_SLACK;
+       k += gridDim.x * blockDim.x) {
+    const uint32_t a = lower_bound_u32(keys, n, k);
+    gp[k] = a;
+    if (k % PAGE_GBXS == 0 && (k < c.ngbxs || k == 0))
+      c.pstart[k / PAGE_GBXS] = a + k / PAGE_GBXS * PAGE_SLACK;
+    if (k == c.ngbxs) {
+      c.pstart[c.npages] = a + c.npages * PAGE_SLACK;
+      const uint32_t out = lower_bound_u32(keys, n, k + 1) - a;
+      c.counters[3] = c.counters[2];
+      c.counters[2] += out;
+    }
   }
 }
-// the in-domain superdroplets (sorted positions j < gp[ngbxs]) into their pages of dst
+// The store from the sorted positions, in one launch of independent parts: the in-domain
+// superdroplets (j < gp[ngbxs]) into their pages of dst, the out-of-domain and null ones (keys ==
+// ngbxs) appended to their store, the pages' free slots, the gridboxes' ranges, the store's ends.
+// (Seven launches before; the free slots, a thread a page, took 110 us on 4096 pages.)
 __global__ void __launch_bounds__(256)
 k_gather_paged(const __grid_constant__ DevCtx c, Fields src, Fields dst,
                const uint32_t* __restrict__ keys, const uint32_t* __restrict__ perm,
                const uint32_t* __restrict__ gp) {
-  const uint32_t nd = gp[c.ngbxs];
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nd; j += gridDim.x * blockDim.x) {
-    const uint32_t p = keys[j] / PAGE_GBXS;
-    copy_rec(src, perm[j], dst, c.pstart[p] + (j - gp[p * PAGE_GBXS]));
-  }
-}
-// holes after each page's superdroplets; the gridboxes' ranges; the store's ends
-__global__ void k_pg_fill_full(const __grid_constant__ DevCtx c, Fields dst,
-                               const uint32_t* __restrict__ gp) {
+  const uint32_t nd = gp[c.ngbxs], nall = gp[c.ngbxs + 1], out0 = c.counters[3];
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-  for (uint32_t p = tid; p < c.npages; p += nt) {
-    const uint32_t lo = p * PAGE_GBXS, hi = min(lo + PAGE_GBXS, c.ngbxs);
-    for (uint32_t o = c.pstart[p] + (gp[hi] - gp[lo]); o < c.pstart[p + 1]; ++o) set_hole(dst, o);
+  for (uint32_t j = tid; j < nall; j += nt) {
+    if (j < nd) {
+      const uint32_t p = keys[j] / PAGE_GBXS;
+      copy_rec(src, perm[j], dst, c.pstart[p] + (j - gp[p * PAGE_GBXS]));
+    } else {
+      copy_rec(src, perm[j], c.grave, out0 + (j - nd));
+    }
   }
+  for (uint32_t h = tid; h < c.npages * PAGE_SLACK; h += nt)
+    set_hole(dst, c.pstart[h / PAGE_SLACK + 1] - PAGE_SLACK + h % PAGE_SLACK);
   for (uint32_t g = tid; g < c.ngbxs; g += nt) {
     const uint32_t p = g / PAGE_GBXS;
     c.gstart[g] = c.pstart[p] + (gp[g] - gp[p * PAGE_GBXS]);
     c.gcount[g] = gp[g + 1] - gp[g];
   }
-}
-// out-of-domain and null superdroplets (sorted keys == ngbxs) appended to the out-of-domain store
-__global__ void k_grave_sorted(const __grid_constant__ DevCtx c, Fields src,
-                               const uint32_t* __restrict__ perm, const uint32_t* __restrict__ gp) {
-  const uint32_t a = gp[c.ngbxs], b = gp[c.ngbxs + 1], ng0 = c.counters[2];
-  for (uint32_t j = a + blockIdx.x * blockDim.x + threadIdx.x; j < b; j += gridDim.x * blockDim.x)
-    copy_rec(src, perm[j], c.grave, ng0 + (j - a));
-}
-__global__ void k_full_commit(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ gp) {
-  const uint32_t total = c.pstart[c.npages];
-  c.counters[2] += gp[c.ngbxs + 1] - gp[c.ngbxs];
-  c.counters[0] = total;
-  c.counters[1] = gp[c.ngbxs];
-  c.gstart[c.ngbxs] = total;
-  c.gstart[c.ngbxs + 1] = total;
+  if (tid == 0) {
+    const uint32_t total = c.pstart[c.npages];
+    c.counters[0] = total;
+    c.counters[1] = nd;
+    c.gstart[c.ngbxs] = total;
+    c.gstart[c.ngbxs + 1] = total;
+  }
 }
 
 // ---- re-sort after motion ----
 // pg_ctr: [0] pages touched, [1] a page outgrows its slots (repack), [2] movers into the
 // out-of-domain store (their first sorted index), [3] the re-sort's stamp (counts re-sorts)
-__global__ void k_pg_reset(const __grid_constant__ DevCtx c) {
-  c.pg_ctr[0] = 0;
-  c.pg_ctr[1] = 0;
-  c.pg_ctr[2] = 0;
-  c.pg_ctr[3] += 1;
-}
-// the movers' records, in their sorted order
-__global__ void __launch_bounds__(256)
-k_mv_gather(const __grid_constant__ DevCtx c, Fields src, const uint32_t* __restrict__ mvp,
-            const uint32_t* __restrict__ m_ptr) {
-  const uint32_t m = *m_ptr;
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x)
-    copy_rec(src, mvp[j], c.mvrec, j);
-}
+// (k_motion resets the first three and counts the fourth up)
 __device__ __forceinline__ void touch_page(const DevCtx& c, uint32_t p) {
   if (atomicExch(&c.pg_flag[p], 1u) == 0u) c.pg_list[atomicAdd(&c.pg_ctr[0], 1u)] = p;
 }
-// the pages movers leave or enter
-__global__ void k_pg_touch(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ mk,
-                           const uint32_t* __restrict__ mvp, const uint32_t* __restrict__ m_ptr) {
-  const uint32_t m = *m_ptr;
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
-    const uint32_t k = mk[j];
-    if (k < c.ngbxs) touch_page(c, k / PAGE_GBXS);
-    touch_page(c, page_of_slot(c, mvp[j]));
-    if (j == 0) c.pg_ctr[2] = lower_bound_u32(mk, m, c.ngbxs);
-  }
-}
-
-// each gridbox's run of sorted movers [mv_lo, mv_hi), stamped with this re-sort's stamp (a
-// gridbox whose stamp is older has no arrivals)
-__global__ void k_mv_runs(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ mk,
-                          const uint32_t* __restrict__ m_ptr) {
+// The sorted movers, a thread each: their records copied out, the pages they leave or enter, each
+// gridbox's run [mv_lo, mv_hi) of them, stamped with this re-sort's stamp (a gridbox whose stamp is
+// older has no arrivals), and those out of the domain (and null ones) appended to their store (its
+// count follows in k_pg_commit).
+__global__ void __launch_bounds__(256)
+k_mv_place(const __grid_constant__ DevCtx c, Fields src, const uint32_t* __restrict__ mk,
+           const uint32_t* __restrict__ mvp, const uint32_t* __restrict__ m_ptr) {
   const uint32_t m = *m_ptr, stamp = c.pg_ctr[3];
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
-    const uint32_t k = mk[j];
-    if (k >= c.ngbxs) continue;
-    if (j == 0 || mk[j - 1] != k) {
-      c.mv_lo[k] = j;
-      c.mv_stamp[k] = stamp;
+    const uint32_t k = mk[j], i = mvp[j];
+    copy_rec(src, i, c.mvrec, j);
+    touch_page(c, page_of_slot(c, i));
+    if (j == 0) c.pg_ctr[2] = lower_bound_u32(mk, m, c.ngbxs);
+    if (k < c.ngbxs) {
+      touch_page(c, k / PAGE_GBXS);
+      if (j == 0 || mk[j - 1] != k) {
+        c.mv_lo[k] = j;
+        c.mv_stamp[k] = stamp;
+      }
+      if (j + 1 == m || mk[j + 1] != k) c.mv_hi[k] = j + 1;
+    } else {
+      copy_rec(src, i, c.grave, c.counters[2] + (j - lower_bound_u32(mk, m, c.ngbxs)));
     }
-    if (j + 1 == m || mk[j + 1] != k) c.mv_hi[k] = j + 1;
   }
 }
 
@@ -397,7 +378,24 @@ k_pg_copy_back(const __grid_constant__ DevCtx c, Fields src, const uint32_t* __r
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
     copy_rec(src, i, c.sd, i);
 }
-__global__ void k_pg_commit(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ pnew) {
+// the new page starts from their sizes, in place (npages + 1 entries), by one block
+__global__ void __launch_bounds__(SCAN_THREADS)
+k_pg_scan(const __grid_constant__ DevCtx c, uint32_t* __restrict__ pnew) {
+  __shared__ uint32_t wsum[32];
+  if (c.pg_ctr[1] == 0) return;
+  uint32_t carry = 0;
+  for (uint32_t p0 = 0; p0 < c.npages; p0 += SCAN_THREADS) {
+    const uint32_t p = p0 + threadIdx.x;
+    uint32_t total;
+    const uint32_t ex =
+        block_exclusive_scan_1024(p < c.npages ? pnew[p] : 0u, wsum, total);
+    if (p < c.npages) pnew[p] = carry + ex;
+    carry += total;
+  }
+  if (threadIdx.x == 0) pnew[c.npages] = carry;
+}
+__global__ void k_pg_commit(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ pnew,
+                            const uint32_t* __restrict__ m_ptr) {
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
   const bool repack = c.pg_ctr[1] != 0;
   if (repack) {
@@ -407,17 +405,8 @@ __global__ void k_pg_commit(const __grid_constant__ DevCtx c, const uint32_t* __
   if (tid == 0) {
     const uint32_t total = repack ? pnew[c.npages] : c.counters[0];
     c.counters[0] = total;
+    c.counters[2] += *m_ptr - c.pg_ctr[2];  // movers into the out-of-domain store
     c.gstart[c.ngbxs] = total;
     c.gstart[c.ngbxs + 1] = total;
   }
-}
-// movers out of the domain (and null ones) appended to the out-of-domain store
-__global__ void k_grave_movers(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ m_ptr) {
-  const uint32_t m = *m_ptr, a = c.pg_ctr[2], ng0 = c.counters[2];
-  for (uint32_t j = a + blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x)
-    copy_rec(c.mvrec, j, c.grave, ng0 + (j - a));
-}
-__global__ void k_grave_movers_commit(const __grid_constant__ DevCtx c,
-                                      const uint32_t* __restrict__ m_ptr) {
-  c.counters[2] += *m_ptr - c.pg_ctr[2];
 }

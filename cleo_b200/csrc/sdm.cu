@@ -27,6 +27,7 @@
 // seeding.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -85,7 +86,8 @@ struct DevCtx {
   uint32_t *mv_scan, *gstart_new;  // mv_scan: movers per 32 slots, scanned (exclusive)
   uint32_t* mv_mask;   // the movers among each 32 slots, a bit each (k_motion)
   uint32_t* mv_tsums;  // the count scan's tile offsets (the scan's readers add them: mv_before)
-  uint32_t* mv_total;  // valid superdroplets that changed gridbox in the last motion step
+  uint32_t* mv_total;  // [0] valid superdroplets that changed gridbox in this motion step, [1] its
+                       // finished blocks; both 0 between steps
   // paged layout (pages.cuh): pages of PAGE_GBXS gridboxes, their slot starts (npages + 1), the
   // touched-page flags and list, the re-sort's counters, the movers' records; slots = the SoA
   // buffers' length (capacity plus the pages' slack)
@@ -125,8 +127,8 @@ struct cleo_b200_ctx {
   int device = 0;
   // sort scratch
   uint32_t *keys[2], *vals[2], *hist, *tile_sums;
-  uint32_t *gs_tsums = nullptr, *mv_count = nullptr;  // scan tile totals, the mover count
-  uint32_t *pstart_new = nullptr, *ps_tsums = nullptr;  // page re-sort: repacked page starts
+  uint32_t* mv_count = nullptr;
+  uint32_t* pstart_new = nullptr;  // page re-sort: repacked page starts
   double* qm_buf = nullptr;  // BatchScratch::qm's storage
   bool one_box = false;      // a one-gridbox domain: collisions by the kernels of onebox.cuh
   OneBox ob{};
@@ -139,6 +141,7 @@ struct cleo_b200_ctx {
   cudaEvent_t ev_report = nullptr;
   bool report_recorded = false;
   bool sort_full = false;
+  bool movers_few = false;  // the previous motion step's movers: the page re-sort's own sort
   bool last_sort_full = false;  // what the last re-sort after motion was (cleo_b200_resort_stats)
   int resort_policy = CLEO_RESORT_AUTO;
   int sms = 148;                // the device's SMs
@@ -216,16 +219,15 @@ struct cleo_b200_ctx {
   const cleo_b200_mlp* mlp = nullptr;
   double* seed_buf = nullptr;
   size_t seed_cap = 0;
-  // two-pass condensation_solve scratch (deferred-solve list and its radix sort)
+  // two-pass condensation_solve scratch: the deferred solves' classes, positions and order
   struct CsScratch {
     size_t cap = 0;
-    uint32_t *k0 = nullptr, *v0 = nullptr, *k1 = nullptr, *v1 = nullptr;
-    uint32_t *hist = nullptr, *tsums = nullptr, *ctr = nullptr;  // ctr: deferred solves
-    double* zres = nullptr;  // pass A's iterates of the restarts
-    uint32_t nt = 0;
+    uint32_t *cls = nullptr, *vals = nullptr, *order = nullptr;
+    uint32_t* ctr = nullptr;  // [0] deferred solves, then COST_CLASSES counts and cursors
+    double* zres = nullptr;   // pass A's iterates of the restarts
   } cs;
   void free_cs() {
-    for (uint32_t* q : {cs.k0, cs.v0, cs.k1, cs.v1, cs.hist, cs.tsums, cs.ctr}) cudaFree(q);
+    for (uint32_t* q : {cs.cls, cs.vals, cs.order, cs.ctr}) cudaFree(q);
     cudaFree(cs.zres);
     cs = CsScratch();
   }
@@ -332,12 +334,11 @@ __device__ __forceinline__ bool beyond_domainboundary(uint32_t gbxindex, uint32_
 // neighbour search, the bounds check); returns whether it moves in the re-sort (changes gridbox,
 // leaves the domain, or is a null one collisions left). For the full sort it writes the sort key
 // (gridbox, ngbxs out of the domain, ngbxs + 1 for a free slot) and position.
-__device__ __forceinline__ bool move_superdroplet(const DevCtx& c, uint32_t i,
+__device__ __forceinline__ bool move_superdroplet(const DevCtx& c, uint32_t i, uint32_t g,
                                                   uint32_t* __restrict__ keys,
                                                   uint32_t* __restrict__ vals, int incremental) {
   const uint32_t ng = c.ngbxs;
   const double delt = c.p.motion_delt;
-  const uint32_t g = c.sd.gbx[i];
   if (!incremental) vals[i] = i;
   if (g >= ng) {  // a null superdroplet left by collisions (out of the domain), or a free slot
     const bool hole = is_hole(c.sd, i);
@@ -345,16 +346,16 @@ __device__ __forceinline__ bool move_superdroplet(const DevCtx& c, uint32_t i,
     return !hole;  // a null one moves to the out-of-domain store
   }
     const Where w{c.err, g, i};
+    const double c3 = c.sd.c3[i], c1 = c.sd.c1[i], c2 = c.sd.c2[i], radius = c.sd.r[i];
     double bzl, bzh, bxl, bxh, byl, byh;
     bounds_of(c.b3lo, c.b3hi, ng, g, bzl, bzh);
     bounds_of(c.b1lo, c.b1hi, ng, g, bxl, bxh);
     bounds_of(c.b2lo, c.b2hi, ng, g, byl, byh);
     const double wl = c.wlo[g], wh = c.whi[g], ul = c.ulo[g], uh = c.uhi[g], vl = c.vlo[g],
                  vh = c.vhi[g];
-    const double c3 = c.sd.c3[i], c1 = c.sd.c1[i], c2 = c.sd.c2[i];
     // delta_coord3: predcorr.hpp:83-105
     double coord3 = c3;
-    const double terminal = terminalv(c.p.motion_tv, c.sd.r[i]);
+    const double terminal = terminalv(c.p.motion_tv, radius);
     double vel3 = interpolation(bzl, bzh, wl, wh, coord3);
     vel3 -= terminal;
     coord3 += vel3 * delt;
@@ -382,8 +383,8 @@ __device__ __forceinline__ bool move_superdroplet(const DevCtx& c, uint32_t i,
     // monitor_precipitation (monitor_precipitation_observer.hpp:97-107): the contribution of a
     // superdroplet below its gridbox's lower bound, added per gridbox in order by k_mon_precip
     if (c.precip_c)
-      c.precip_c[i] = (n3 < bzl) ? condensate_mass(c.sd.r[i], c.sd.msol[i], w) *
-                                       (double)c.sd.xi[i] / Rho_l / c.gbxarea[g]
+      c.precip_c[i] = (n3 < bzl) ? condensate_mass(radius, c.sd.msol[i], w) * (double)c.sd.xi[i] /
+                                       Rho_l / c.gbxarea[g]
                                  : 0.0;
     // change_if_coord3nghbr: finite z, coordinate unchanged at the edge (cartesianmaps.cpp:184-213)
     uint32_t idx = g;
@@ -472,16 +473,30 @@ __device__ __forceinline__ bool move_superdroplet(const DevCtx& c, uint32_t i,
     }
     return mover;
 }
-__global__ void __launch_bounds__(256, 4)  // 64 registers: measured 15% faster than 80
-k_motion(const __grid_constant__ DevCtx c, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, int incremental) {
+// A resident grid walks the slots (so few blocks count down at the end); the gridbox index, behind
+// which the gridbox's twelve values wait, is loaded a slot ahead.
+constexpr int MOTION_THREADS = 256, MOTION_CTAS = 4;  // 64 registers: 15% faster than 80
+__global__ void __launch_bounds__(MOTION_THREADS, MOTION_CTAS)
+k_motion(const __grid_constant__ DevCtx c, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+         uint32_t* __restrict__ report, int incremental) {
   const uint32_t n = c.counters[0];
   const uint32_t nchunks = (n + 31) / 32;
-  if (incremental && blockIdx.x == 0 && threadIdx.x == 0) c.mv_scan[nchunks] = 0;  // scan total
+  if (incremental && blockIdx.x == 0 && threadIdx.x == 0) {
+    c.mv_scan[nchunks] = 0;  // scan total
+    // the page re-sort's counters (pages.cuh), which nothing reads before its kernels
+    c.pg_ctr[0] = c.pg_ctr[1] = c.pg_ctr[2] = 0;
+    c.pg_ctr[3] += 1;
+  }
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
   // i0 is the same for the whole block, so every warp's lanes cover 32 consecutive slots together
-  for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
-    const uint32_t i = i0 + threadIdx.x;
+  uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x;
+  uint32_t g_next = i0 + threadIdx.x < n ? c.sd.gbx[i0 + threadIdx.x] : OOB;
+  for (; i0 < n; i0 += step) {
+    const uint32_t i = (uint32_t)i0 + threadIdx.x;
+    const uint32_t g = g_next;
+    g_next = i0 + step + threadIdx.x < n ? c.sd.gbx[i0 + step + threadIdx.x] : OOB;
     bool mover = false;
-    if (i < n) mover = move_superdroplet(c, i, keys, vals, incremental);
+    if (i < n) mover = move_superdroplet(c, i, g, keys, vals, incremental);
     if (incremental) {  // the movers of the warp's 32 slots: a mask and its count
       const unsigned bm = __ballot_sync(0xFFFFFFFFu, mover);
       if ((threadIdx.x & 31) == 0 && i < n) {
@@ -490,10 +505,18 @@ k_motion(const __grid_constant__ DevCtx c, uint32_t* __restrict__ keys, uint32_t
       }
     }
   }
-}
-__global__ void k_mv_report(const __grid_constant__ DevCtx c, uint32_t* __restrict__ out) {  // mapped host memory
-  out[0] = *c.mv_total;
-  out[1] = c.counters[0];
+  // the last block reports {movers, slots} to the host (mapped memory; an event behind this kernel
+  // marks it) and clears the two counters for the next step: a memory-set node cost 4 us of a
+  // graph's step, a kernel of its own 1.5
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&c.mv_total[1], 1u) == gridDim.x - 1) {
+      report[0] = atomicExch(&c.mv_total[0], 0u);
+      report[1] = n;
+      c.mv_total[1] = 0;
+    }
+  }
 }
 
 // ---- the movers of a page re-sort (pages.cuh), listed in position order ----
@@ -505,8 +528,10 @@ __device__ __forceinline__ uint32_t mv_before(const DevCtx& c, uint32_t w) {
 }
 // the movers, from the masks of the chunks that hold any: positions and keys (min(gbx, ngbxs) of
 // the gridbox indices k_motion wrote)
-__global__ void k_mv_list(const __grid_constant__ DevCtx c, uint32_t* __restrict__ mk, uint32_t* __restrict__ mvp) {
+__global__ void k_mv_list(const __grid_constant__ DevCtx c, uint32_t* __restrict__ mk,
+                          uint32_t* __restrict__ mvp, uint32_t* __restrict__ count) {
   const uint32_t nchunks = (c.counters[0] + 31) / 32;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *count = mv_before(c, nchunks);  // number of movers
   for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < nchunks;
        w += gridDim.x * blockDim.x) {
     uint32_t m = c.mv_mask[w];
@@ -521,9 +546,6 @@ __global__ void k_mv_list(const __grid_constant__ DevCtx c, uint32_t* __restrict
       ++p;
     }
   }
-}
-__global__ void k_mv_count(const __grid_constant__ DevCtx c, uint32_t* __restrict__ count) {
-  *count = mv_before(c, (c.counters[0] + 31) / 32);  // number of movers
 }
 // ---- superdroplet output: the domain superdroplets, gathered in gridbox order and converted
 // the way the reference's Collect* functors convert them (superdrops_observer.hpp:139-464) ----
@@ -921,8 +943,7 @@ namespace {
 // Two-pass form of the batch solve (the batched schedule), as k_cond_a / k_cond_b do for the
 // SDM step: pass A finishes every direct solve that converges within its first two iterations
 // (or within the seeded attempt) and lists the rest, keyed by sub-step count; pass B solves the
-// listed ones after the list has been sorted by that key, so that neighbouring lanes carry
-// similar work. Iterations spent in pass A on an abandoned seed are carried in niters_out.
+// listed ones by cost class (k_cond_place), so that neighbouring lanes carry similar work. Iterations spent in pass A on an abandoned seed are carried in niters_out.
 __device__ __forceinline__ uint32_t cs_warp_append(uint32_t* ctr, bool flag) {
   const unsigned m = __ballot_sync(0xFFFFFFFFu, flag);
   uint32_t base = 0;
@@ -939,6 +960,9 @@ k_cs_a(const __grid_constant__ DevCtx c, uint32_t n, const double* __restrict__ 
        double* __restrict__ zres, uint32_t* __restrict__ lkeys, uint32_t* __restrict__ lvals,
        uint32_t* __restrict__ ctr) {
   const NewtonCfg cfg{c.p.maxniters, c.p.rtol, c.p.atol};
+  __shared__ uint32_t cnt[COST_CLASSES];
+  class_count_begin(cnt);
+  uint32_t restarts = 0;
   for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
     const uint32_t i = i0 + threadIdx.x;
     bool defer = false;
@@ -981,7 +1005,7 @@ k_cs_a(const __grid_constant__ DevCtx c, uint32_t n, const double* __restrict__ 
         }
       } else {
         defer = true;
-        key = deferred_key(dt, fmax(crit, c.p.cond_minsubdelt), true);
+        key = cost_class(dt, fmax(crit, c.p.cond_minsubdelt));
       }
       if (defer && niters_out) niters_out[i] = carried | (failed ? CLEO_NITERS_FAILED : 0u);
     }
@@ -990,7 +1014,9 @@ k_cs_a(const __grid_constant__ DevCtx c, uint32_t n, const double* __restrict__ 
       lkeys[pos] = key;
       lvals[pos] = i;
     }
+    class_count(cnt, restarts, defer, key);
   }
+  class_count_end(cnt, restarts, ctr + 1);
 }
 __global__ void __launch_bounds__(256)
 k_cs_b(const __grid_constant__ DevCtx c, const double* __restrict__ radius, const double* __restrict__ msol,
@@ -998,14 +1024,13 @@ k_cs_b(const __grid_constant__ DevCtx c, const double* __restrict__ radius, cons
        const double* __restrict__ s_ratio, const double* __restrict__ delt,
        const double* __restrict__ seeds, double* __restrict__ out,
        uint32_t* __restrict__ niters_out, const double* __restrict__ zres,
-       const uint32_t* __restrict__ lkeys, const uint32_t* __restrict__ lvals,
-       const uint32_t* __restrict__ ctr) {
+       const uint32_t* __restrict__ order, const uint32_t* __restrict__ ctr) {
   const NewtonCfg cfg{c.p.maxniters, c.p.rtol, c.p.atol};
-  const uint32_t nl = *ctr;
+  const uint32_t nl = ctr[0], restarts = ctr[1];
   for (uint32_t jr = blockIdx.x * blockDim.x + threadIdx.x; jr < nl;
        jr += gridDim.x * blockDim.x) {
     const uint32_t j = nl - 1 - jr;  // most expensive solves first (the list is sorted by cost)
-    const uint32_t i = lvals[j];
+    const uint32_t i = order[j];
     uint32_t failed = 0;
     const Where w{c.err, OOB, i, &failed};
     const double T = temp[i], r = radius[i], dt = delt[i];
@@ -1015,8 +1040,8 @@ k_cs_b(const __grid_constant__ DevCtx c, const double* __restrict__ radius, cons
     kohler_factors(msol[i], T, akoh, bkoh);
     uint32_t ni = 0;
     double newr;
-    const double zr = lkeys[j] == 0u ? zres[i] : 0.0;
-    if (lkeys[j] == 0u && cfg.maxniters >= 2 && zr == zr) {
+    const double zr = j < restarts ? zres[i] : 0.0;
+    if (j < restarts && cfg.maxniters >= 2 && zr == zr) {
       // a direct solve whose two reference iterations in pass A did not converge: the restart
       // continues from them (resume_restart)
       const OdeConsts o = ode_consts(s_ratio[i], akoh, bkoh, ffactor / ventilation_factor(r));
@@ -1074,6 +1099,12 @@ int grid_for(size_t n, int threads) {
   return (int)b;
 }
 
+// blocks of k_cond_place for a list of up to n solves, whose count only the device knows
+int place_grid(size_t n, int sms) {
+  const size_t b = (n + PLACE_ITEMS - 1) / PLACE_ITEMS;
+  return (int)std::min<size_t>(b ? b : 1, (size_t)sms * 8);
+}
+
 // exclusive scan of a[0, n) on the context's stream, in place, the total into a[n] (tsums: the
 // scan's tile totals, (n + SCAN_TILE) / SCAN_TILE + 1 words)
 void scan_u32(cleo_b200_ctx* x, uint32_t* a, uint32_t n, uint32_t* tsums) {
@@ -1092,47 +1123,22 @@ void scan_u32(cleo_b200_ctx* x, uint32_t* a, uint32_t n, uint32_t* tsums) {
 int sort_current(cleo_b200_ctx* x) {
   DevCtx& d = x->d;
   cudaStream_t s = x->stream;
-  const uint32_t nt = x->ntiles_max;
-  uint32_t* kin = x->keys[0];
-  uint32_t* vin = x->vals[0];
-  uint32_t* kout = x->keys[1];
-  uint32_t* vout = x->vals[1];
-  const uint64_t nh = (uint64_t)256 * nt;
-  const uint32_t nscan_tiles = (uint32_t)((nh + SCAN_TILE - 1) / SCAN_TILE);
-  for (uint32_t shift = 0; shift < x->key_bits; shift += 8) {
-    k_rs_upsweep<<<nt, RS_THREADS, 0, s>>>(kin, d.counters, (int)shift, x->hist, nt);
-    k_scan_tiles<<<nscan_tiles, SCAN_THREADS, 0, s>>>(x->hist, x->hist, nh, x->tile_sums);
-    k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(x->tile_sums, nscan_tiles, nullptr);
-    k_scan_add<<<(unsigned)((nh + 255) / 256), 256, 0, s>>>(x->hist, nh, x->tile_sums);
-    k_rs_downsweep<<<nt, RS_THREADS, 0, s>>>(kin, vin, d.counters, (int)shift, x->hist, nt, kout,
-                                             vout);
-    x->launches += 5;
-    std::swap(kin, kout);
-    std::swap(vin, vout);
-  }
-  // sorted (key, position) now in kin/vin
+  const int r = radix_passes(s, x->keys[0], x->vals[0], x->keys[0], x->vals[0], x->keys[1],
+                             x->vals[1], nullptr, d.counters, 0, x->key_bits, x->hist,
+                             x->tile_sums, x->ntiles_max, 0, 0xFFFFFFFFu, &x->launches);
+  // sorted (key, position)
+  const uint32_t *kin = x->keys[r], *vin = x->vals[r];
   Fields& src = x->buf[x->cur];
   Fields& dst = x->buf[1 - x->cur];
   uint32_t* gp = d.gstart_new;
-  const int gs = grid_for(d.slots, 256), gp2 = grid_for((size_t)d.ngbxs + 2, 256);
-  k_lower_bounds<<<gp2, 256, 0, s>>>(d, kin, gp);
-  k_pg_sizes_full<<<grid_for(d.npages, 256), 256, 0, s>>>(d, gp, d.pstart);
+  k_lower_bounds<<<grid_for((size_t)d.ngbxs + 2, 256), 256, 0, s>>>(d, kin, gp);
+  k_gather_paged<<<grid_for(d.slots, 256), 256, 0, s>>>(d, src, dst, kin, vin, gp);
   x->launches += 2;
-  scan_u32(x, d.pstart, d.npages, x->ps_tsums);
-  k_gather_paged<<<gs, 256, 0, s>>>(d, src, dst, kin, vin, gp);
-  k_pg_fill_full<<<grid_for(std::max(d.npages, d.ngbxs), 256), 256, 0, s>>>(d, dst, gp);
-  k_grave_sorted<<<gs, 256, 0, s>>>(d, src, vin, gp);
-  k_full_commit<<<1, 1, 0, s>>>(d, gp);
-  x->launches += 4;
   x->cur = 1 - x->cur;
   d.sd = x->buf[x->cur];
   CUDA_TRY(cudaGetLastError());
   return CLEO_OK;
 }
-
-int radix_pairs_on(cleo_b200_ctx* x, uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1,
-                   const uint32_t* n_ptr, uint32_t bits, uint32_t* hist, uint32_t* tile_sums,
-                   uint32_t nt, uint32_t unsorted_max = 0);
 
 // The page re-sort after motion (pages.cuh; k_motion left a mover mask per 32 slots): scan of the
 // masks' counts, the movers listed in position order and stably radix-sorted by key, copied out
@@ -1148,16 +1154,23 @@ int sort_incremental(cleo_b200_ctx* x) {
   // reads) (readers add the tile offsets: mv_before)
   const uint64_t n1 = ((uint64_t)d.slots + 31) / 32 + 1;
   const uint32_t nscan = (uint32_t)((n1 + SCAN_TILE - 1) / SCAN_TILE);
-  k_pg_reset<<<1, 1, 0, s>>>(d);
   k_scan_tiles<<<nscan, SCAN_THREADS, 0, s>>>(d.mv_scan, d.mv_scan, n1, d.mv_tsums);
   k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(d.mv_tsums, nscan, nullptr);
+  k_mv_list<<<grid_for(n1, 256), 256, 0, s>>>(d, x->keys[1], x->vals[1], x->mv_count);
   x->launches += 3;
-  k_mv_list<<<grid_for(n1, 256), 256, 0, s>>>(d, x->keys[1], x->vals[1]);
-  k_mv_count<<<1, 1, 0, s>>>(d, x->mv_count);
-  x->launches += 2;
-  // the movers stably by key (the mover count is read by the radix kernels on the device)
-  const int where = radix_pairs_on(x, x->keys[1], x->vals[1], d.scr_p, d.scr_j, x->mv_count,
-                                   x->key_bits, x->hist, x->tile_sums, x->ntiles_max);
+  // the movers stably by key: up to RS_SMALL_MAX in one block; more by the multi-tile passes, which
+  // are only launched (their kernels return at once when they are not needed, 1.3 us each) when
+  // the last step's movers were not few; a step that then has many all the same stays with the block
+  const bool few = x->movers_few;
+  k_rs_small<<<1, RS_SMALL_THREADS, 0, s>>>(x->keys[1], x->vals[1], x->keys[1], x->vals[1], d.scr_p,
+                                            d.scr_j, nullptr, x->mv_count, 0, x->key_bits,
+                                            few ? 1 : 0, 0xFFFFFFFFu);
+  x->launches += 1;
+  int where = (int)(x->key_bits / 8 & 1);
+  if (!few)
+    where = radix_passes(s, x->keys[1], x->vals[1], x->keys[1], x->vals[1], d.scr_p, d.scr_j,
+                         nullptr, x->mv_count, 0, x->key_bits, x->hist, x->tile_sums,
+                         x->ntiles_max, RS_SMALL_MAX, 0xFFFFFFFFu, &x->launches);
   const uint32_t* mk = where == 0 ? x->keys[1] : d.scr_p;
   const uint32_t* mvp = where == 0 ? x->vals[1] : d.scr_j;
   const int pgrid = 148 * 8;  // CTAs over the touched pages (persistent loop)
@@ -1165,62 +1178,18 @@ int sort_incremental(cleo_b200_ctx* x) {
   Fields& other = x->buf[1 - x->cur];
   // grid-stride kernels over the movers, whose count only the device knows: one wave of CTAs
   const int mgrid = 148 * 8;
-  k_mv_gather<<<mgrid, 256, 0, s>>>(d, cur, mvp, x->mv_count);
-  k_pg_touch<<<mgrid, 256, 0, s>>>(d, mk, mvp, x->mv_count);
-  k_mv_runs<<<mgrid, 256, 0, s>>>(d, mk, x->mv_count);
+  k_mv_place<<<mgrid, 256, 0, s>>>(d, cur, mk, mvp, x->mv_count);
   k_pg_plan<<<pgrid, 256, 0, s>>>(d, mk, mvp, x->mv_count);
-  k_grave_movers<<<mgrid, 256, 0, s>>>(d, x->mv_count);
-  k_grave_movers_commit<<<1, 1, 0, s>>>(d, x->mv_count);
   k_pg_write<false><<<pgrid, 256, 0, s>>>(d, cur, mk, mvp, x->mv_count, d.pstart);
-  x->launches += 7;
   // the repack path: its kernels return at once unless k_pg_plan chose it
   k_pg_sizes_repack<<<pgrid, 256, 0, s>>>(d, mk, mvp, x->mv_count, x->pstart_new);
-  x->launches += 1;
-  scan_u32(x, x->pstart_new, d.npages, x->ps_tsums);
+  k_pg_scan<<<1, SCAN_THREADS, 0, s>>>(d, x->pstart_new);
   k_pg_write<true><<<pgrid, 256, 0, s>>>(d, other, mk, mvp, x->mv_count, x->pstart_new);
   k_pg_copy_back<<<mgrid, 256, 0, s>>>(d, other, x->pstart_new);
-  k_pg_commit<<<grid_for((size_t)d.npages + 1, 256), 256, 0, s>>>(d, x->pstart_new);
-  x->launches += 3;
+  k_pg_commit<<<grid_for((size_t)d.npages + 1, 256), 256, 0, s>>>(d, x->pstart_new, x->mv_count);
+  x->launches += 8;
   CUDA_TRY(cudaGetLastError());
   return CLEO_OK;
-}
-
-// stable radix sort of (key, value) pairs whose count is *n_ptr (device), over `bits` key bits,
-// from (k0, v0) using (k1, v1) as the other buffer; returns 0 if the result is in (k0, v0)
-// with explicit digit-table scratch for nt tiles (hist: 256 nt words, tile_sums: enough for the
-// scan of the table)
-int radix_pairs_on(cleo_b200_ctx* x, uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1,
-                   const uint32_t* n_ptr, uint32_t bits, uint32_t* hist, uint32_t* tile_sums,
-                   uint32_t nt, uint32_t unsorted_max) {
-  cudaStream_t s = x->stream;
-  const uint64_t nh = (uint64_t)256 * nt;
-  const uint32_t nscan_tiles = (uint32_t)((nh + SCAN_TILE - 1) / SCAN_TILE);
-  int cur = 0;
-  uint32_t* K[2] = {k0, k1};
-  uint32_t* V[2] = {v0, v1};
-  // counts up to RS_SMALL_MAX (the usual mover list) are sorted by one block; the multi-tile passes
-  // below then return at once, and the other way round
-  // (with unsorted_max, counts up to it stay as they are: a caller for whom the order is only a
-  // schedule, and an even number of passes, so that the sorted result would be in place too)
-  k_rs_small<<<1, RS_SMALL_THREADS, 0, s>>>(k0, v0, k1, v1, n_ptr, bits, unsorted_max);
-  x->launches += 1;
-  constexpr uint32_t SMALL = RS_SMALL_MAX;
-  for (uint32_t shift = 0; shift < bits; shift += 8) {
-    k_rs_upsweep<<<nt, RS_THREADS, 0, s>>>(K[cur], n_ptr, (int)shift, hist, nt, SMALL);
-    k_scan_tiles<<<nscan_tiles, SCAN_THREADS, 0, s>>>(hist, hist, nh, tile_sums, n_ptr, SMALL);
-    k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(tile_sums, nscan_tiles, nullptr, n_ptr, SMALL);
-    k_scan_add<<<(unsigned)((nh + 255) / 256), 256, 0, s>>>(hist, nh, tile_sums, n_ptr, SMALL);
-    k_rs_downsweep<<<nt, RS_THREADS, 0, s>>>(K[cur], V[cur], n_ptr, (int)shift, hist, nt,
-                                             K[1 - cur], V[1 - cur], SMALL);
-    x->launches += 5;
-    cur = 1 - cur;
-  }
-  return cur;
-}
-int radix_pairs(cleo_b200_ctx* x, uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1,
-                const uint32_t* n_ptr, uint32_t bits, uint32_t unsorted_max = 0) {
-  return radix_pairs_on(x, k0, v0, k1, v1, n_ptr, bits, x->hist, x->tile_sums, x->ntiles_max,
-                        unsorted_max);
 }
 
 // the microphysics of one SDM step on the batched schedule (batched.cuh)
@@ -1244,9 +1213,11 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
   b.qm = nullptr;
   BatchScratch bq = b;  // the first sub-step's scratch
   bq.qm = fuse_qcond ? x->qm_buf : nullptr;
-  // every gridbox's RNG slot from 0 at the step's start (a one-gridbox domain's was reset by the
-  // previous step's k_b_advance_t, or at creation)
-  if (!x->one_box) {
+  // every gridbox's RNG slot from 0 at the step's start, by the first condensation sub-step's
+  // k_b_thermo when it starts the step (a one-gridbox domain's was reset by the previous step's
+  // k_b_advance_t, or at creation)
+  const bool thermo_first = on_step(d.p.condstep, t_sdm);
+  if (!x->one_box && !thermo_first) {
     k_b_reset<<<gg, 256, 0, s>>>(d, b, 1);
     x->launches += 1;
   }
@@ -1258,30 +1229,29 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
     if (cond) {
       StageMark mc(x, 3);
       const BatchScratch& bc = subt == t_sdm ? bq : b;  // qcond with the first sub-step's commit
-      k_b_thermo<<<gg, 256, 0, s>>>(d, b);
+      k_b_thermo<<<gg, 256, 0, s>>>(d, b, subt == t_sdm && !x->one_box ? 1 : 0);
       x->launches += 1;
-      if (x->cfg.cond_minb == 5)
-        k_cond_a<5><<<grid_for(d.slots, x->cfg.cond_block), x->cfg.cond_block, 0, s>>>(d, bc);
-      else if (x->cfg.cond_minb == 4)
-        k_cond_a<4><<<grid_for(d.slots, x->cfg.cond_block), x->cfg.cond_block, 0, s>>>(d, bc);
+      const int block = x->cfg.cond_block, minb = x->cfg.cond_minb;
+      const int ga = std::min(x->sms * minb * (256 / block), (int)grid_for(d.slots, block));
+      if (minb == 5)
+        k_cond_a<5><<<ga, block, 0, s>>>(d, bc);
+      else if (minb == 4)
+        k_cond_a<4><<<ga, block, 0, s>>>(d, bc);
       else
-        k_cond_a<3><<<grid_for(d.slots, x->cfg.cond_block), x->cfg.cond_block, 0, s>>>(d, bc);
+        k_cond_a<3><<<ga, block, 0, s>>>(d, bc);
       x->launches += 1;
-      // 16 key bits: two passes, result back in place. The order (most expensive solves first)
-      // balances pass B's load; a list of up to RS_SMALL_MAX solves runs at once on pass B's
-      // resident threads whatever its order, so it stays unsorted, unless the surrogate needs
-      // its restarts at the front
-      const uint32_t unsorted_max = d.p.nr_seed == CLEO_NRSEED_MLP ? 0u : RS_SMALL_MAX;
-      const int where =
-          radix_pairs(x, b.lkeys, b.lvals, x->keys[1], x->vals[1], b.ctr, 16, unsorted_max);
-      if (where != 0) return CLEO_ERR_CUDA;
+      // the deferred solves by cost class: neighbouring lanes carry similar work, the most expensive
+      // start first, and the restarts the surrogate seeds lead
+      k_cond_place<<<place_grid(d.slots, x->sms), 256, 0, s>>>(b.ctr, b.lkeys, b.lvals, b.ccnt,
+                                                              b.order);
+      x->launches += 1;
       if (d.p.nr_seed == CLEO_NRSEED_MLP) {
         // the surrogate seeds only the direct solves pass A left unconverged, in b.dm
         mlp::Infer w;
         if (cleo_mlp_infer_view(x->mlp, &w) != CLEO_OK) return CLEO_ERR_MLP;
         w.err = reinterpret_cast<uint32_t*>(&d.err->code);
         const SdmListSeedIO io{d.sd.gbx, d.sd.r,  d.sd.msol, d.temp, d.press, b.th_s,
-                               d.p.cond_delt, b.lvals, b.ctr + 9, b.dm};
+                               d.p.cond_delt, b.order, b.ccnt, b.dm};
         const uint32_t tiles = (d.slots + mlp::TILE_M - 1) / mlp::TILE_M;
         mlp::k_mlp_tc<SdmListSeedIO><<<tiles < mlp::TC_GRID_MAX ? tiles : mlp::TC_GRID_MAX, 128, mlp::TC_SMEM,
                                        s>>>(w, io, d.slots);
@@ -1378,10 +1348,9 @@ int run_sdm_step(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next) {
     {
       StageMark m(x, 0);
       const bool inc = !x->sort_full;
-      CUDA_TRY(cudaMemsetAsync(d.mv_total, 0, 4, s));
-      k_motion<<<grid_for(d.slots, 256), 256, 0, s>>>(d, x->keys[0], x->vals[0], inc ? 1 : 0);
-      k_mv_report<<<1, 1, 0, s>>>(d, x->d_motion);
-      x->launches += 2;
+      k_motion<<<std::min(x->sms * MOTION_CTAS, grid_for(d.slots, MOTION_THREADS)),
+                 MOTION_THREADS, 0, s>>>(d, x->keys[0], x->vals[0], x->d_motion, inc ? 1 : 0);
+      x->launches += 1;
       {  // inside a captured step the record becomes an external event node of the graph
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         CUDA_TRY(cudaStreamIsCapturing(s, &cs));
@@ -1507,7 +1476,7 @@ int run_step_graphed(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next) {
   const cleo_b200_params& p = x->d.p;
   std::vector<uint32_t> sig;
   sig.push_back((uint32_t)x->cur);
-  sig.push_back((on_step(p.motionstep, t_sdm) ? 1u : 0u) | (x->sort_full ? 2u : 0u));
+  sig.push_back((on_step(p.motionstep, t_sdm) ? 1u : 0u) | (x->sort_full ? 2u : (x->movers_few ? 4u : 0u)));
   sig.push_back(t_sdm_next - t_sdm);
   for (uint32_t subt = t_sdm; subt < t_sdm_next;
        subt = min(next_step(p.condstep, subt), next_step(p.collstep, subt))) {
@@ -1613,7 +1582,6 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   rc |= dalloc(x, &d.mv_hi, d.ngbxs);
   rc |= dalloc(x, &d.mv_stamp, d.ngbxs);
   rc |= dalloc(x, &x->pstart_new, (size_t)d.npages + 1);
-  rc |= dalloc(x, &x->ps_tsums, ((size_t)d.npages + SCAN_TILE) / SCAN_TILE + 1);
   rc |= dalloc(x, &d.gstart, ng + 2);
   rc |= dalloc(x, &d.gcount, ng);
   rc |= dalloc(x, &d.counters, 4);
@@ -1656,6 +1624,8 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   rc |= dalloc(x, &x->bs.ffv, cap);
   rc |= dalloc(x, &x->bs.lkeys, cap);
   rc |= dalloc(x, &x->bs.lvals, cap);
+  rc |= dalloc(x, &x->bs.order, cap);
+  rc |= dalloc(x, &x->bs.ccnt, 2 * COST_CLASSES);
   rc |= dalloc(x, &x->bs.bucket, 4 * ng);
   rc |= dalloc(x, &x->bs.big, ng);
   rc |= dalloc(x, &x->bs.brec, 2 * ng);
@@ -1667,7 +1637,7 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   rc |= dalloc(x, &x->tile_sums, ((size_t)256 * x->ntiles_max + SCAN_TILE - 1) / SCAN_TILE + 1);
   rc |= dalloc(x, &d.mv_scan, ((size_t)cap + 31) / 32 + 1);
   rc |= dalloc(x, &d.mv_mask, ((size_t)cap + 31) / 32);
-  rc |= dalloc(x, &d.mv_total, 1);
+  rc |= dalloc(x, &d.mv_total, 2);
   if (cudaHostAlloc(&x->h_motion, 2 * sizeof(uint32_t), cudaHostAllocMapped) != cudaSuccess ||
       cudaHostGetDevicePointer(&x->d_motion, x->h_motion, 0) != cudaSuccess ||
       cudaEventCreateWithFlags(&x->ev_report, cudaEventDisableTiming) != cudaSuccess)
@@ -1676,11 +1646,7 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
     x->h_motion[0] = x->h_motion[1] = 0;
   rc |= dalloc(x, &d.gstart_new, (size_t)ng + 2);
   rc |= dalloc(x, &x->mv_count, 1);
-  {
-    const size_t a = ((size_t)cap + 1 + SCAN_TILE - 1) / SCAN_TILE, b = ((size_t)ng + SCAN_TILE) / SCAN_TILE;
-    rc |= dalloc(x, &d.mv_tsums, a + 1);
-    rc |= dalloc(x, &x->gs_tsums, b + 1);
-  }
+  rc |= dalloc(x, &d.mv_tsums, ((size_t)cap + SCAN_TILE) / SCAN_TILE + 1);
   if (params->monitors) {
     for (int r = 0; r < 2; ++r) {
       for (int w = 0; w < 2; ++w) {
@@ -1725,6 +1691,7 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   CUDA_TRY(cudaMemsetAsync(d.cond_mass, 0, ng * 8, x->stream));
   CUDA_TRY(cudaMemsetAsync(d.nr_iters, 0, ng * 8, x->stream));
   CUDA_TRY(cudaMemsetAsync(d.counters, 0, 16, x->stream));
+  CUDA_TRY(cudaMemsetAsync(d.mv_total, 0, 8, x->stream));
   CUDA_TRY(cudaMemsetAsync(d.gstart, 0, (ng + 2) * 4, x->stream));
   CUDA_TRY(cudaMemsetAsync(d.gcount, 0, (ng ? ng : 1) * 4, x->stream));
   CUDA_TRY(cudaMemsetAsync(d.pstart, 0, ((size_t)d.npages + 1) * 4, x->stream));
@@ -2035,6 +2002,7 @@ int cleo_b200_step(cleo_b200_ctx* x, uint32_t t_mdl, uint32_t t_next) {
       if (x->report_recorded) CUDA_TRY(cudaEventSynchronize(x->ev_report));
       const volatile uint32_t* hm = x->h_motion;
       const uint32_t movers = hm[0], nsd = hm[1];
+      x->movers_few = x->report_recorded && movers <= RS_SMALL_MAX / 2;
       x->sort_full = x->resort_policy == CLEO_RESORT_FULL ||
                      (x->resort_policy == CLEO_RESORT_AUTO &&
                       ((uint64_t)movers * 5 > (uint64_t)nsd || x->d.npages < (uint32_t)x->sms));
@@ -2398,20 +2366,16 @@ int cleo_b200_condensation_solve(cleo_b200_ctx* x, size_t n, const double* d_rad
     CUDA_TRY(cudaGetLastError());
     return CLEO_OK;
   }
-  // two-pass form: scratch for the deferred list of up to n solves and its 16-bit radix sort
+  // two-pass form: scratch for the deferred list of up to n solves
   auto& cs = x->cs;
+  constexpr size_t CTR_BYTES = (1 + 2 * COST_CLASSES) * sizeof(uint32_t);
   if (n > cs.cap) {
     CUDA_TRY(cudaStreamSynchronize(x->stream));
     x->free_cs();
-    const uint32_t nt = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
-    const uint64_t nh = (uint64_t)256 * nt;
-    const size_t nsums = (size_t)((nh + SCAN_TILE - 1) / SCAN_TILE) + 1;
     bool ok = true;
-    for (uint32_t** q : {&cs.k0, &cs.v0, &cs.k1, &cs.v1})
+    for (uint32_t** q : {&cs.cls, &cs.vals, &cs.order})
       ok = ok && cudaMalloc(q, n * sizeof(uint32_t)) == cudaSuccess;
-    ok = ok && cudaMalloc(&cs.hist, nh * sizeof(uint32_t)) == cudaSuccess;
-    ok = ok && cudaMalloc(&cs.tsums, nsums * sizeof(uint32_t)) == cudaSuccess;
-    ok = ok && cudaMalloc(&cs.ctr, sizeof(uint32_t)) == cudaSuccess;
+    ok = ok && cudaMalloc(&cs.ctr, CTR_BYTES) == cudaSuccess;
     ok = ok && cudaMalloc(&cs.zres, n * sizeof(double)) == cudaSuccess;
     if (!ok) {
       x->free_cs();
@@ -2419,20 +2383,17 @@ int cleo_b200_condensation_solve(cleo_b200_ctx* x, size_t n, const double* d_rad
       return CLEO_ERR_CUDA;
     }
     cs.cap = n;
-    cs.nt = nt;
   }
-  CUDA_TRY(cudaMemsetAsync(cs.ctr, 0, sizeof(uint32_t), x->stream));
+  CUDA_TRY(cudaMemsetAsync(cs.ctr, 0, CTR_BYTES, x->stream));
   k_cs_a<<<grid_for(n, 256), 256, 0, x->stream>>>(
       x->d, (uint32_t)n, d_radius, d_msol, d_temp, d_press, d_s_ratio, d_delt,
-      seeded ? x->seed_buf : nullptr, d_radius_out, d_niters_out, cs.zres, cs.k0, cs.v0, cs.ctr);
-  x->launches += 1;
-  const int where = radix_pairs_on(x, cs.k0, cs.v0, cs.k1, cs.v1, cs.ctr, 16, cs.hist, cs.tsums,
-                                   cs.nt);
-  if (where != 0) return CLEO_ERR_CUDA;  // two 8-bit passes leave the result in (k0, v0)
+      seeded ? x->seed_buf : nullptr, d_radius_out, d_niters_out, cs.zres, cs.cls, cs.vals, cs.ctr);
+  k_cond_place<<<place_grid(n, x->sms), 256, 0, x->stream>>>(cs.ctr, cs.cls, cs.vals, cs.ctr + 1,
+                                                            cs.order);
   k_cs_b<<<x->grid_flat * 2, 256, 0, x->stream>>>(x->d, d_radius, d_msol, d_temp, d_press,
                                                   d_s_ratio, d_delt, seeds, d_radius_out,
-                                                  d_niters_out, cs.zres, cs.k0, cs.v0, cs.ctr);
-  x->launches += 1;
+                                                  d_niters_out, cs.zres, cs.order, cs.ctr);
+  x->launches += 3;
   CUDA_TRY(cudaGetLastError());
   return CLEO_OK;
 }

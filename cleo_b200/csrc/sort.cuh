@@ -4,9 +4,12 @@
 // histogram of sdgbxindex (out-of-domain keys share the last bucket), an exclusive scan and a
 // scatter with atomic_fetch_add, which is stable only on the Serial backend. Here the scatter is
 // made stable on the GPU by a least-significant-digit radix sort of (key, position) pairs with
-// 8-bit digits: per digit pass, every tile of 4096 keys counts its digits (upsweep), the
-// digit-major table of tile counts is scanned, and each tile ranks its keys stably with warp
-// match/ballot (downsweep). No block waits on another block.
+// 8-bit digits: per digit pass, every tile of 4096 keys counts its digits (upsweep), the table of
+// tile counts is scanned, and each tile ranks its keys stably with warp match/ballot (downsweep).
+// No block waits on another block. A pass is two launches for up to RS_SELF_TILES tiles (each
+// downsweep block adds the table up itself), three while the scan's tile totals are few enough for
+// a block to add up (RS_RAW_SUMS), else four: on small sorts a launch costs as much as its work
+// (about 1.2 us in a graph beside 2 us of run time; 5 launches a pass before).
 #pragma once
 
 #include <cstdint>
@@ -21,53 +24,118 @@ constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
-// per-tile digit counts; hist is digit-major: hist[d * ntiles + tile]. With small_n > 0 the
-// pass does nothing for n <= small_n (k_rs_small sorts those in one block).
+constexpr uint32_t RS_SELF_TILES = 64;
+constexpr uint32_t RS_RAW_SUMS = 64;
+
+// per-tile digit counts: hist[d * ntiles + tile], or hist[tile * 256 + d] for SELF. With small_n
+// > 0 the pass does nothing for n <= small_n (k_rs_small sorts those in one block). Keys above
+// `cap` count as cap.
+template <bool SELF>
 __global__ void __launch_bounds__(RS_THREADS)
-k_rs_upsweep(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ n_ptr, int shift,
-             uint32_t* __restrict__ hist, uint32_t ntiles, uint32_t small_n = 0) {
+k_rs_upsweep(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ n_ptr, uint32_t n_val,
+             int shift, uint32_t* __restrict__ hist, uint32_t ntiles, uint32_t small_n,
+             uint32_t cap) {
   __shared__ uint32_t cnt[256];
-  const uint32_t n = *n_ptr;
+  const uint32_t n = n_ptr ? *n_ptr : n_val;
   if (small_n > 0 && n <= small_n) return;
   for (int i = threadIdx.x; i < 256; i += RS_THREADS) cnt[i] = 0;
   __syncthreads();
   const uint32_t tile = blockIdx.x;
   const uint64_t base = (uint64_t)tile * RS_TILE;
+  // all loads first; then one shared atomic per digit a warp meets: the keys are nearly sorted, so
+  // a warp's are mostly one digit, and 32 atomics on it would run one after another
+  uint32_t dg[RS_ITEMS];
 #pragma unroll
   for (int k = 0; k < RS_ITEMS; ++k) {
     const uint64_t idx = base + (uint64_t)k * RS_THREADS + threadIdx.x;
-    if (idx < n) atomicAdd(&cnt[(keys[idx] >> shift) & 255u], 1u);
+    dg[k] = idx < n ? (min(keys[idx], cap) >> shift) & 255u : 256u;
+  }
+#pragma unroll
+  for (int k = 0; k < RS_ITEMS; ++k) {
+    const unsigned peers = __match_any_sync(0xFFFFFFFFu, dg[k]);
+    if (dg[k] < 256u && (int)(threadIdx.x & 31) == __ffs(peers) - 1)
+      atomicAdd(&cnt[dg[k]], (uint32_t)__popc(peers));
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 256; i += RS_THREADS) hist[(uint64_t)i * ntiles + tile] = cnt[i];
+  for (int i = threadIdx.x; i < 256; i += RS_THREADS)
+    hist[SELF ? (uint64_t)tile * 256 + i : (uint64_t)i * ntiles + tile] = cnt[i];
 }
 
-// stable scatter of one digit pass
+// stable scatter of one digit pass. offs: the counts (SELF), or their scan within scan tiles, with
+// the scan tiles' totals in tsums, exclusively scanned or (raw_sums) as they are. vin may be null:
+// a value is then its position.
+template <bool SELF>
 __global__ void __launch_bounds__(RS_THREADS)
 k_rs_downsweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-               const uint32_t* __restrict__ n_ptr, int shift, const uint32_t* __restrict__ offs,
-               uint32_t ntiles, uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
-               uint32_t small_n = 0) {
+               const uint32_t* __restrict__ n_ptr, uint32_t n_val, int shift,
+               const uint32_t* __restrict__ offs,
+               uint32_t ntiles, const uint32_t* __restrict__ tsums, uint32_t raw_sums,
+               uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t small_n,
+               uint32_t cap) {
   __shared__ uint32_t wcount[RS_WARPS][256];
   __shared__ uint32_t dbase[256];
-  const uint32_t n = *n_ptr;
+  __shared__ uint32_t pre[RS_RAW_SUMS];
+  const uint32_t n = n_ptr ? *n_ptr : n_val;
   const uint32_t tile = blockIdx.x;
   const uint64_t base = (uint64_t)tile * RS_TILE;
   if (base >= n || (small_n > 0 && n <= small_n)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) (&wcount[0][0])[i] = 0;
-  for (int i = threadIdx.x; i < 256; i += RS_THREADS) dbase[i] = offs[(uint64_t)i * ntiles + tile];
+  if constexpr (SELF) {
+    // digit d = thread: the tiles' counts of it before this one, and in all
+    const uint32_t d = threadIdx.x;
+    uint32_t before = 0, total = 0;
+#pragma unroll 8
+    for (uint32_t t = 0; t < ntiles; ++t) {
+      const uint32_t c = offs[t * 256 + d];
+      before += t < tile ? c : 0u;
+      total += c;
+    }
+    uint32_t x = total;  // exclusive scan of the digits' totals
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) pre[warp] = x;
+    __syncthreads();
+    uint32_t w0 = 0;
+    for (int w = 0; w < warp; ++w) w0 += pre[w];
+    dbase[d] = w0 + x - total + before;
+  } else {
+    if (raw_sums > 0) {
+      if (warp == 0) {  // up to 64 totals: two a lane
+        const uint32_t i = 2 * lane;
+        const uint32_t a = i < raw_sums ? tsums[i] : 0u;
+        const uint32_t b = i + 1 < raw_sums ? tsums[i + 1] : 0u;
+        uint32_t x = a + b;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+          if (lane >= o) x += y;
+        }
+        pre[i] = x - a - b;
+        pre[i + 1] = x - b;
+      }
+      __syncthreads();
+    }
+    for (int i = threadIdx.x; i < 256; i += RS_THREADS) {
+      const uint64_t e = (uint64_t)i * ntiles + tile;
+      dbase[i] = offs[e] + (raw_sums > 0 ? pre[e / SCAN_TILE] : tsums[e / SCAN_TILE]);
+    }
+  }
   __syncthreads();
   const unsigned lt = (1u << lane) - 1u;
   uint32_t kk[RS_ITEMS], vv[RS_ITEMS], rk[RS_ITEMS];
   // warp w owns the contiguous chunk [w*32*ITEMS, (w+1)*32*ITEMS) of the tile, read in rounds of
-  // 32 consecutive keys: rank order = array order
+  // 32 consecutive keys: rank order = array order (loading all of them first takes 93 registers for
+  // 80 and was slower where there are many tiles: 80 us a pass for 50 on 6.6 M keys)
 #pragma unroll
   for (int j = 0; j < RS_ITEMS; ++j) {
     const uint64_t idx = base + (uint64_t)warp * 32 * RS_ITEMS + (uint64_t)j * 32 + lane;
     const bool valid = idx < n;
-    kk[j] = valid ? kin[idx] : 0u;
-    vv[j] = valid ? vin[idx] : 0u;
+    kk[j] = valid ? min(kin[idx], cap) : 0u;
+    vv[j] = valid ? (vin ? vin[idx] : (uint32_t)idx) : 0u;
     const uint32_t d = valid ? ((kk[j] >> shift) & 255u) : 256u;
     const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
     const int leader = __ffs(peers) - 1;
@@ -100,84 +168,108 @@ k_rs_downsweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vi
   }
 }
 
-// The same stable LSD sort for n <= RS_SMALL_MAX pairs (device count) in one block of
-// RS_SMALL_THREADS: `bits` key bits in 8-bit passes between (k0, v0) and (k1, v1), leaving the
-// result where the multi-tile passes would (in (k0, v0) after an even number of passes). Returns
-// at once for larger n, which the multi-tile passes sort.
+// The same stable LSD sort in one block of RS_SMALL_THREADS, for counts (on the device) up to
+// RS_SMALL_MAX: `bits` key bits in 8-bit passes between (k0, v0) and (k1, v1), leaving the result
+// where the multi-tile passes would (in (k0, v0) after an even number of passes). Returns at once
+// for larger n, which the multi-tile passes sort, unless `any` is set: then it takes them too, tile
+// after tile (a caller that expects few and launches no other passes; about 12 us a tile of 16384
+// and pass). The first pass's values may be positions (v_first null), its keys capped.
 constexpr int RS_SMALL_THREADS = 1024;
 constexpr int RS_SMALL_WARPS = RS_SMALL_THREADS / 32;
 constexpr uint32_t RS_SMALL_MAX = (uint32_t)RS_SMALL_THREADS * RS_ITEMS;  // 16384
 __global__ void __launch_bounds__(RS_SMALL_THREADS)
-k_rs_small(uint32_t* __restrict__ k0, uint32_t* __restrict__ v0, uint32_t* __restrict__ k1,
-           uint32_t* __restrict__ v1, const uint32_t* __restrict__ n_ptr, uint32_t bits,
-           uint32_t unsorted_max = 0) {
+k_rs_small(const uint32_t* k_first, const uint32_t* v_first, uint32_t* k0, uint32_t* v0,
+           uint32_t* k1, uint32_t* v1, uint32_t* v_last, const uint32_t* __restrict__ n_ptr,
+           uint32_t n_val, uint32_t bits, int any, uint32_t cap) {
   __shared__ uint32_t wcount[RS_SMALL_WARPS][256];
   __shared__ uint32_t dbase[256];
   __shared__ uint32_t wsum[8];
-  const uint32_t n = *n_ptr;
-  if (n > RS_SMALL_MAX || n <= unsorted_max) return;
+  const uint32_t n = n_ptr ? *n_ptr : n_val;
+  if (n > RS_SMALL_MAX && !any) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
+  const uint32_t d = threadIdx.x;  // digit of the threads below 256
   uint32_t* K[2] = {k0, k1};
   uint32_t* V[2] = {v0, v1};
   int cur = 0;
   for (uint32_t shift = 0; shift < bits; shift += 8) {
-    for (int i = threadIdx.x; i < RS_SMALL_WARPS * 256; i += RS_SMALL_THREADS)
-      (&wcount[0][0])[i] = 0;
-    __syncthreads();
-    uint32_t kk[RS_ITEMS], vv[RS_ITEMS], rk[RS_ITEMS];
+    const uint32_t* kin = shift == 0 ? k_first : K[cur];
+    const uint32_t* vin = shift == 0 ? v_first : V[cur];
+    if (n > RS_SMALL_MAX) {  // the digits' counts over all tiles
+      if (d < 256) dbase[d] = 0;
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < n; i += RS_SMALL_THREADS)
+        atomicAdd(&dbase[(min(kin[i], cap) >> shift) & 255u], 1u);
+      __syncthreads();
+    }
+    for (uint32_t t0 = 0; t0 < n || t0 == 0; t0 += RS_SMALL_MAX) {
+      for (int i = threadIdx.x; i < RS_SMALL_WARPS * 256; i += RS_SMALL_THREADS)
+        (&wcount[0][0])[i] = 0;
+      __syncthreads();
+      uint32_t kk[RS_ITEMS], vv[RS_ITEMS], rk[RS_ITEMS];
 #pragma unroll
-    for (int j = 0; j < RS_ITEMS; ++j) {  // array order = rank order, as in k_rs_downsweep
-      const uint32_t idx = (uint32_t)warp * 32 * RS_ITEMS + (uint32_t)j * 32 + lane;
-      const bool valid = idx < n;
-      kk[j] = valid ? K[cur][idx] : 0u;
-      vv[j] = valid ? V[cur][idx] : 0u;
-      const uint32_t d = valid ? ((kk[j] >> shift) & 255u) : 256u;
-      const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
-      const int leader = __ffs(peers) - 1;
-      uint32_t prev = 0;
-      if (valid) prev = wcount[warp][d];
-      __syncwarp();
-      if (valid && lane == leader) wcount[warp][d] = prev + __popc(peers);
-      __syncwarp();
-      rk[j] = valid ? (prev + __popc(peers & lt)) : 0xFFFFFFFFu;
-    }
-    __syncthreads();
-    // digit d = thread d < 256: its per-warp offsets, then the exclusive scan of the digit totals
-    // over the first 8 warps
-    const uint32_t d = threadIdx.x;
-    uint32_t tot = 0, x = 0;
-    if (d < 256) {
-      for (int w = 0; w < RS_SMALL_WARPS; ++w) {
-        const uint32_t c = wcount[w][d];
-        wcount[w][d] = tot;
-        tot += c;
+      for (int j = 0; j < RS_ITEMS; ++j) {  // array order = rank order, as in k_rs_downsweep
+        const uint32_t idx = t0 + (uint32_t)warp * 32 * RS_ITEMS + (uint32_t)j * 32 + lane;
+        const bool valid = idx < n;
+        kk[j] = valid ? min(kin[idx], cap) : 0u;
+        vv[j] = valid ? (vin ? vin[idx] : idx) : 0u;
+        rk[j] = 0xFFFFFFFFu;
       }
-      x = tot;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= o) x += y;
+      for (int j = 0; j < RS_ITEMS; ++j) {
+        const bool valid = t0 + (uint32_t)warp * 32 * RS_ITEMS + (uint32_t)j * 32 + lane < n;
+        if (t0 + (uint32_t)warp * 32 * RS_ITEMS + (uint32_t)j * 32 >= n) continue;  // whole warp
+        const uint32_t dg = valid ? ((kk[j] >> shift) & 255u) : 256u;
+        const unsigned peers = __match_any_sync(0xFFFFFFFFu, dg);
+        const int leader = __ffs(peers) - 1;
+        uint32_t prev = 0;
+        if (valid) prev = wcount[warp][dg];
+        __syncwarp();
+        if (valid && lane == leader) wcount[warp][dg] = prev + __popc(peers);
+        __syncwarp();
+        if (valid) rk[j] = prev + __popc(peers & lt);
       }
-      if (lane == 31) wsum[warp] = x;
-    }
-    __syncthreads();
-    if (d < 256) {
-      uint32_t before = 0;
-      for (int w = 0; w < warp; ++w) before += wsum[w];
-      dbase[d] = before + x - tot;
-    }
-    __syncthreads();
+      __syncthreads();
+      // the per-warp offsets of a digit, then (first tile) the exclusive scan of the digits' totals
+      // over the first 8 warps
+      uint32_t tot = 0, x = 0, all = 0;
+      if (d < 256) {
+#pragma unroll 8
+        for (int w = 0; w < RS_SMALL_WARPS; ++w) {
+          const uint32_t c = wcount[w][d];
+          wcount[w][d] = tot;
+          tot += c;
+        }
+        all = n > RS_SMALL_MAX ? dbase[d] : tot;
+        x = all;
 #pragma unroll
-    for (int j = 0; j < RS_ITEMS; ++j) {
-      if (rk[j] != 0xFFFFFFFFu) {
-        const uint32_t dg = (kk[j] >> shift) & 255u;
-        const uint32_t pos = dbase[dg] + wcount[warp][dg] + rk[j];
-        K[1 - cur][pos] = kk[j];
-        V[1 - cur][pos] = vv[j];
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+          if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[warp] = x;
       }
+      __syncthreads();
+      if (d < 256 && t0 == 0) {
+        uint32_t before = 0;
+        for (int w = 0; w < warp; ++w) before += wsum[w];
+        dbase[d] = before + x - all;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < RS_ITEMS; ++j) {
+        if (rk[j] != 0xFFFFFFFFu) {
+          const uint32_t dg = (kk[j] >> shift) & 255u;
+          const uint32_t pos = dbase[dg] + wcount[warp][dg] + rk[j];
+          K[1 - cur][pos] = kk[j];
+          (v_last && shift + 8 >= bits ? v_last : V[1 - cur])[pos] = vv[j];
+        }
+      }
+      __syncthreads();  // this tile's writes before the next pass reads them
+      if (d < 256) dbase[d] += tot;  // the next tile's digits follow
+      if (n <= RS_SMALL_MAX) break;
+      __syncthreads();
     }
-    __syncthreads();  // this pass's writes before the next pass reads them
     cur ^= 1;
   }
 }
@@ -261,6 +353,50 @@ __global__ void k_scan_add(uint32_t* __restrict__ out, uint64_t n,
   if (gate && *gate <= gate_max) return;
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] += tile_sums[i / SCAN_TILE];
+}
+
+// The count of pairs is *n_ptr on the device, or n_val where n_ptr is null; k_rs_small and
+// radix_passes write the last pass's values to v_last where it is given.
+// Stable radix sort of (key, value) pairs over `bits` key bits
+// (8-bit passes), for up to nt tiles: reads (k_first, v_first) (v_first null: positions; keys
+// capped), then uses the buffers (k0, v0) and (k1, v1) in turn, the first pass writing (k1, v1).
+// Returns 0 if the result is in (k0, v0), else 1. hist: 256 nt words; tsums: their scan's tile
+// totals. With small_n the passes do nothing for counts up to it. Adds its launches to *launches.
+inline int radix_passes(cudaStream_t s, const uint32_t* k_first, const uint32_t* v_first,
+                        uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1,
+                        uint32_t* v_last, const uint32_t* n_ptr, uint32_t n_val, uint32_t bits,
+                        uint32_t* hist, uint32_t* tsums,
+                        uint32_t nt, uint32_t small_n, uint32_t cap,
+                        unsigned long long* launches) {
+  const uint64_t nh = (uint64_t)256 * nt;
+  const uint32_t nscan = (uint32_t)((nh + SCAN_TILE - 1) / SCAN_TILE);
+  uint32_t* K[2] = {k0, k1};
+  uint32_t* V[2] = {v0, v1};
+  int cur = 0;
+  for (uint32_t shift = 0; shift < bits; shift += 8) {
+    const uint32_t* kin = shift == 0 ? k_first : K[cur];
+    const uint32_t* vin = shift == 0 ? v_first : V[cur];
+    uint32_t* vout = v_last && shift + 8 >= bits ? v_last : V[1 - cur];
+    if (nt <= RS_SELF_TILES) {
+      k_rs_upsweep<true><<<nt, RS_THREADS, 0, s>>>(kin, n_ptr, n_val, (int)shift, hist, nt, small_n,
+                                                      cap);
+      k_rs_downsweep<true><<<nt, RS_THREADS, 0, s>>>(kin, vin, n_ptr, n_val, (int)shift, hist, nt, tsums,
+                                                     0, K[1 - cur], vout, small_n, cap);
+      *launches += 2;
+    } else {
+      const bool raw = nscan <= RS_RAW_SUMS;
+      k_rs_upsweep<false><<<nt, RS_THREADS, 0, s>>>(kin, n_ptr, n_val, (int)shift, hist, nt, small_n,
+                                                      cap);
+      k_scan_tiles<<<nscan, SCAN_THREADS, 0, s>>>(hist, hist, nh, tsums, n_ptr, small_n);
+      if (!raw) k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(tsums, nscan, nullptr, n_ptr, small_n);
+      k_rs_downsweep<false><<<nt, RS_THREADS, 0, s>>>(kin, vin, n_ptr, n_val, (int)shift, hist, nt, tsums,
+                                                      raw ? nscan : 0, K[1 - cur], vout,
+                                                      small_n, cap);
+      *launches += raw ? 3 : 4;
+    }
+    cur = 1 - cur;
+  }
+  return cur;
 }
 
 }  // namespace cleo

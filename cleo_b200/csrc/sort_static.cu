@@ -29,15 +29,14 @@ constexpr uint32_t SORT_STATIC_MAX = 1u << 20;  // superdroplets per call
 constexpr uint32_t TILES_MAX = (SORT_STATIC_MAX + cleo::RS_TILE - 1) / cleo::RS_TILE;
 constexpr uint32_t HIST_MAX = 256 * TILES_MAX;
 constexpr uint32_t SCAN_SUMS_MAX = (HIST_MAX + cleo::SCAN_TILE - 1) / cleo::SCAN_TILE + 1;
-// layout (u32 words): keys[2][MAX], vals[2][MAX], hist[HIST_MAX], scan sums, n
+// layout (u32 words): keys[2][MAX], vals[2][MAX], hist[HIST_MAX], scan sums
 constexpr size_t OFF_KEYS0 = 0;
 constexpr size_t OFF_KEYS1 = OFF_KEYS0 + SORT_STATIC_MAX;
 constexpr size_t OFF_VALS0 = OFF_KEYS1 + SORT_STATIC_MAX;
 constexpr size_t OFF_VALS1 = OFF_VALS0 + SORT_STATIC_MAX;
 constexpr size_t OFF_HIST = OFF_VALS1 + SORT_STATIC_MAX;
 constexpr size_t OFF_SUMS = OFF_HIST + HIST_MAX;
-constexpr size_t OFF_N = OFF_SUMS + SCAN_SUMS_MAX;
-constexpr size_t SCRATCH_WORDS = OFF_N + 64;
+constexpr size_t SCRATCH_WORDS = OFF_SUMS + SCAN_SUMS_MAX + 64;
 constexpr size_t SCRATCH_BYTES = SCRATCH_WORDS * sizeof(uint32_t);
 static_assert(SCRATCH_BYTES < (17u << 20), "the static scratch stays under 17 MiB");
 
@@ -49,26 +48,10 @@ constexpr int MAX_DEVICES = 64;
 std::mutex g_setup_mutex;
 uint32_t* g_scratch_ptr[MAX_DEVICES] = {};
 
-// keys = min(sdgbxindex, ngbxs) (out-of-domain keys share the last bucket, sortsupers.hpp:44-48)
-__global__ void k_static_keys(const uint32_t* __restrict__ gbx, uint32_t n, uint32_t ngbxs,
-                              uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                              uint32_t* __restrict__ n_slot) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) *n_slot = n;
-  if (i < n) {
-    const uint32_t g = gbx[i];
-    keys[i] = g < ngbxs ? g : ngbxs;
-    vals[i] = i;
-  }
-}
-
-__global__ void k_static_out(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
-                             uint32_t n, uint32_t ngbxs, uint32_t* __restrict__ order,
+// gstart[k] = first sorted position with key >= k, k = 0 .. ngbxs + 1
+__global__ void k_static_out(const uint32_t* __restrict__ keys, uint32_t n, uint32_t ngbxs,
                              uint32_t* __restrict__ gstart) {
   const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) order[j] = vals[j];
-  if (!gstart) return;
-  // gstart[k] = first sorted position with key >= k, k = 0 .. ngbxs + 1
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < ngbxs + 2; k += stride) {
     uint32_t lo = 0, len = n;
     while (len > 0) {
@@ -130,29 +113,38 @@ extern "C" int cleo_b200_sort_by_gridbox_static(const uint32_t* d_sdgbxindex, ui
   uint32_t* vals[2] = {base + OFF_VALS0, base + OFF_VALS1};
   uint32_t* hist = base + OFF_HIST;
   uint32_t* sums = base + OFF_SUMS;
-  uint32_t* n_slot = base + OFF_N;
-  // every word the passes read is written first in this call (keys/vals for [0, n), the whole
-  // digit table by the upsweep), so nothing left by an earlier call needs clearing
-  k_static_keys<<<(n + 255) / 256, 256, 0, s>>>(d_sdgbxindex, n, ngbxs, keys[0], vals[0], n_slot);
+  // every word the passes read is written first in this call (the whole digit table by the
+  // upsweep), so nothing left by an earlier call needs clearing
   uint32_t bits = 0;
   while (bits < 32 && (((uint64_t)1 << bits) <= (uint64_t)ngbxs)) ++bits;
   const uint32_t key_bits = bits == 0 ? 8 : ((bits + 7) / 8) * 8;
   const uint32_t nt = (n + cleo::RS_TILE - 1) / cleo::RS_TILE;
-  const uint64_t nh = (uint64_t)256 * nt;
-  const uint32_t nscan = (uint32_t)((nh + cleo::SCAN_TILE - 1) / cleo::SCAN_TILE);
-  int cur = 0;
-  for (uint32_t shift = 0; shift < key_bits; shift += 8) {
-    cleo::k_rs_upsweep<<<nt, cleo::RS_THREADS, 0, s>>>(keys[cur], n_slot, (int)shift, hist, nt);
-    cleo::k_scan_tiles<<<nscan, cleo::SCAN_THREADS, 0, s>>>(hist, hist, nh, sums);
-    cleo::k_scan_sums<<<1, cleo::SCAN_THREADS, 0, s>>>(sums, nscan, nullptr);
-    cleo::k_scan_add<<<(unsigned)((nh + 255) / 256), 256, 0, s>>>(hist, nh, sums);
-    cleo::k_rs_downsweep<<<nt, cleo::RS_THREADS, 0, s>>>(keys[cur], vals[cur], n_slot, (int)shift,
-                                                         hist, nt, keys[1 - cur], vals[1 - cur]);
-    cur = 1 - cur;
+  // The first pass reads the gridbox indices themselves (capped: out-of-domain keys share the last
+  // bucket, sortsupers.hpp:44-48) and its positions, the last writes the caller's order. The host's
+  launches bound the call: 1,000,003 superdroplets on 32,768 gridboxes, 12 launches 78 us, now 7
+  // (52 us); up to RS_SMALL_MAX, one block sorts them in one launch.
+  // (One pass that overwrites its own input goes through the scratch instead.)
+  const uint32_t passes = key_bits / 8;
+  const bool in_place = passes == 1 && d_order < d_sdgbxindex + n && d_sdgbxindex < d_order + n;
+  uint32_t* v_last = in_place ? nullptr : d_order;
+  unsigned long long launches = 0;
+  int cur;
+  if (n <= cleo::RS_SMALL_MAX) {
+    cleo::k_rs_small<<<1, cleo::RS_SMALL_THREADS, 0, s>>>(d_sdgbxindex, nullptr, keys[0], vals[0],
+                                                          keys[1], vals[1], v_last, nullptr, n,
+                                                          key_bits, 0, ngbxs);
+    cur = (int)(passes & 1);
+  } else {
+    cur = cleo::radix_passes(s, d_sdgbxindex, nullptr, keys[0], vals[0], keys[1], vals[1], v_last,
+                             nullptr, n, key_bits, hist, sums, nt, 0, ngbxs, &launches);
   }
-  const uint32_t outn = n > ngbxs + 2 ? n : ngbxs + 2;
-  unsigned blocks = (outn + 255) / 256;
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  k_static_out<<<blocks, 256, 0, s>>>(keys[cur], vals[cur], n, ngbxs, d_order, d_gstart);
+  if (in_place && cudaMemcpyAsync(d_order, vals[cur], (size_t)n * 4, cudaMemcpyDeviceToDevice, s) !=
+                      cudaSuccess)
+    return CLEO_ERR_CUDA;
+  if (d_gstart) {
+    unsigned blocks = (ngbxs + 2 + 255) / 256;
+    if (blocks > 148 * 32) blocks = 148 * 32;
+    k_static_out<<<blocks, 256, 0, s>>>(keys[cur], n, ngbxs, d_gstart);
+  }
   return cudaGetLastError() == cudaSuccess ? CLEO_OK : CLEO_ERR_CUDA;
 }
