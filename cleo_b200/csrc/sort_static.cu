@@ -121,7 +121,7 @@ extern "C" int cleo_b200_sort_by_gridbox_static(const uint32_t* d_sdgbxindex, ui
   const uint32_t nt = (n + cleo::RS_TILE - 1) / cleo::RS_TILE;
   // The first pass reads the gridbox indices themselves (capped: out-of-domain keys share the last
   // bucket, sortsupers.hpp:44-48) and its positions, the last writes the caller's order. The host's
-  launches bound the call: 1,000,003 superdroplets on 32,768 gridboxes, 12 launches 78 us, now 7
+  // launches bound the call: 1,000,003 superdroplets on 32,768 gridboxes, 12 launches 78 us, now 7
   // (52 us); up to RS_SMALL_MAX, one block sorts them in one launch.
   // (One pass that overwrites its own input goes through the scratch instead.)
   const uint32_t passes = key_bits / 8;
