@@ -65,7 +65,10 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want) {
 // terms of gridbox g0 + j's valid superdroplets [gstart, gstart + gcount) one after another: the
 // reference's sequential loop (seq_sum's order). Each window starts at the first element a lane
 // still has to add, so ranges no lane adds are not read, and is loaded into registers while the
-// window before it is being added. With skip_big, a gridbox of more than
+// window before it is being added. On smaller domains a warp takes fewer gridboxes (seq_per), down
+// to one: a window's additions are a chain, and 32 gridboxes a warp left two warps a scheduler on
+// 50 thousand gridboxes (a mass-moment call 59 us, now 45; 4096 gridboxes' commit 25 us, now 8).
+// With skip_big, a gridbox of more than
 // SEQ_BIG superdroplets is left out (its lane adds nothing): warp_seq_sums sums it with a warp of
 // its own, so that one long sequential sum does not hold up its batch and large gridboxes are
 // summed in parallel.
@@ -76,7 +79,8 @@ template <class Term, class Iters>
 __device__ __forceinline__ void warp_batch_sums(const DevCtx& c, uint32_t g0, uint32_t nb,
                                                 double* dbuf, uint32_t* ubuf, Term term,
                                                 Iters iters, double& sum,
-                                                unsigned long long& its, bool skip_big) {
+                                                unsigned long long& its, bool skip_big,
+                                                double init = 0.0) {
   constexpr int PER = SEQ_WIN / 32;  // elements of a window per lane
   constexpr uint32_t NONE = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31;
@@ -85,7 +89,7 @@ __device__ __forceinline__ void warp_batch_sums(const DevCtx& c, uint32_t g0, ui
   const uint32_t s = own ? c.gstart[g0 + lane] : hi;
   uint32_t e = own ? s + c.gcount[g0 + lane] : hi;
   if (skip_big && e - s > SEQ_BIG) e = s;
-  double acc = 0.0;
+  double acc = init;
   unsigned long long it = 0;
   uint32_t cur = s;  // this lane's next element to add
   // the window [w0, w0 + SEQ_WIN) clipped to hi, loaded into registers a window ahead
@@ -179,14 +183,16 @@ __device__ __forceinline__ void set_qcond(const DevCtx& c, uint32_t g, double m)
   const double rho_cond = m / c.volume[g] * R0cubed_VOL0;
   c.qcond[g] = rho_cond / dry_air_density(c.press[g], c.temp[g], c.qvap[g]);
 }
-__global__ void __launch_bounds__(SEQ_THREADS) k_b_qcond(const __grid_constant__ DevCtx c) {
+// per: gridboxes of a warp (seq_per)
+__global__ void __launch_bounds__(SEQ_THREADS) k_b_qcond(const __grid_constant__ DevCtx c,
+                                                         uint32_t per) {
   __shared__ double dbuf[SEQ_THREADS / 32][SEQ_WIN];
   __shared__ uint32_t ubuf[SEQ_THREADS / 32][SEQ_WIN];
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (uint32_t g0 = warp * 32; g0 < c.ngbxs; g0 += nwarps * 32) {
-    const uint32_t nb = c.ngbxs - g0 < 32 ? c.ngbxs - g0 : 32;
+  for (uint32_t g0 = warp * per; g0 < c.ngbxs; g0 += nwarps * per) {
+    const uint32_t nb = c.ngbxs - g0 < per ? c.ngbxs - g0 : per;
     double m;
     unsigned long long unused;
     warp_batch_sums(
@@ -486,14 +492,14 @@ __device__ __forceinline__ void cond_commit(const DevCtx& c, uint32_t g, double 
 // reference's sequential reduction, condensation.cpp:29-35), their Newton iterations, then the
 // state update (cond_commit). Empty gridboxes commit a zero change, as the reference's do.
 // Gridboxes of more than SEQ_BIG superdroplets are listed for k_b_commit_big instead.
-__global__ void __launch_bounds__(SEQ_THREADS) k_b_commit(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b) {
+__global__ void __launch_bounds__(SEQ_THREADS) k_b_commit(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b, uint32_t per) {
   __shared__ double dbuf[SEQ_THREADS / 32][SEQ_WIN];
   __shared__ uint32_t ubuf[SEQ_THREADS / 32][SEQ_WIN];
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (uint32_t g0 = warp * 32; g0 < c.ngbxs; g0 += nwarps * 32) {
-    const uint32_t nb = c.ngbxs - g0 < 32 ? c.ngbxs - g0 : 32;
+  for (uint32_t g0 = warp * per; g0 < c.ngbxs; g0 += nwarps * per) {
+    const uint32_t nb = c.ngbxs - g0 < per ? c.ngbxs - g0 : per;
     const bool own = (uint32_t)lane < nb;
     const bool big = own && c.gcount[g0 + lane] > SEQ_BIG;
     const uint32_t pos = warp_append(&b.ctr[10], big);
@@ -513,14 +519,14 @@ __global__ void __launch_bounds__(SEQ_THREADS) k_b_commit(const __grid_constant_
     if (own && !big) cond_commit(c, g0 + lane, m, it);
   }
 }
-// the listed gridboxes of more than SEQ_BIG superdroplets, a warp each (the same sums and
-// updates as k_b_commit's lanes make)
-__global__ void __launch_bounds__(SEQ_THREADS) k_b_commit_big(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b) {
+// the listed gridboxes of more than SEQ_BIG superdroplets, or all of a domain with few (`all`; then
+// k_b_commit is not launched), a warp each (the same sums and updates as k_b_commit's lanes make)
+__global__ void __launch_bounds__(SEQ_THREADS) k_b_commit_big(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b, int all) {
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t nbig = b.ctr[10];
+  const uint32_t nbig = all ? c.ngbxs : b.ctr[10];
   for (uint32_t j = warp; j < nbig; j += nwarps) {
-    const uint32_t g = b.big[j];
+    const uint32_t g = all ? j : b.big[j];
     const uint32_t s = c.gstart[g], e = s + c.gcount[g];
     double mq, md;
     unsigned long long it;

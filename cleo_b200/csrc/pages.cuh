@@ -160,7 +160,8 @@ k_mv_place(const __grid_constant__ DevCtx c, Fields src, const uint32_t* __restr
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
     const uint32_t k = mk[j], i = mvp[j];
     copy_rec(src, i, c.mvrec, j);
-    touch_page(c, page_of_slot(c, i));
+    const uint32_t page = c.mv_page[i];
+    touch_page(c, page != OOB ? page : page_of_slot(c, i));
     if (j == 0) c.pg_ctr[2] = lower_bound_u32(mk, m, c.ngbxs);
     if (k < c.ngbxs) {
       touch_page(c, k / PAGE_GBXS);
@@ -174,6 +175,11 @@ k_mv_place(const __grid_constant__ DevCtx c, Fields src, const uint32_t* __restr
     }
   }
 }
+
+// Threads of the kernels that take a page per CTA: a warp's gridboxes of the page, a chain of
+// dependent loads each, run one after another, so few touched pages (the usual case) are bound by
+// their number: 4 a warp, 8 before (the planning pass 15 us, the writing pass 34; now 10 and 26).
+constexpr int PG_THREADS = 512;
 
 // One page's new content, worked out by a CTA: per gridbox (a warp each) its stayers counted and
 // the sorted movers into it, split at its old start (plan_page); then where each gridbox goes
@@ -216,10 +222,11 @@ __device__ void plan_page(const DevCtx& c, uint32_t p, const uint32_t* mvp, Page
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (warp == 0) {
     uint32_t s = 0;
-    for (uint32_t q = 0; q < ng; ++q) s += pl.ns[q] + pl.na[q];
-    pl.total = s;
+    for (uint32_t q = lane; q < ng; q += 32) s += pl.ns[q] + pl.na[q];
+    s = __reduce_add_sync(0xFFFFFFFFu, s);
+    if (lane == 0) pl.total = s;
   }
   __syncthreads();
 }
@@ -230,27 +237,44 @@ __device__ void plan_page(const DevCtx& c, uint32_t p, const uint32_t* mvp, Page
 // when superdroplets left or entered it or its start moved; the others stay where they are.
 __device__ void place_page(const DevCtx& c, uint32_t p, uint32_t pbase, uint32_t pend, bool keep,
                            PagePlan& pl) {
-  if (threadIdx.x == 0) {
-    const uint32_t ng = min(PAGE_GBXS, c.ngbxs - p * PAGE_GBXS);
-    bool fits = false;
-    if (keep) {
-      uint32_t e = pbase;
-      for (uint32_t q = 0; q < ng; ++q) {
-        const uint32_t s = max(pl.b[q], e);
-        pl.st[q] = s;
-        e = s + pl.ns[q] + pl.na[q];
-      }
-      fits = e <= pend;
+  if (threadIdx.x < 32) {  // a warp, two gridboxes a lane
+    static_assert(PAGE_GBXS == 64, "two gridboxes a lane");
+    const uint32_t ng = min(PAGE_GBXS, c.ngbxs - p * PAGE_GBXS), lane = threadIdx.x;
+    const uint32_t q0 = 2 * lane, q1 = q0 + 1;
+    const uint32_t n0 = q0 < ng ? pl.ns[q0] + pl.na[q0] : 0u;
+    const uint32_t n1 = q1 < ng ? pl.ns[q1] + pl.na[q1] : 0u;
+    uint32_t x = n0 + n1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if ((int)lane >= o) x += y;
     }
-    if (!fits) {
-      uint32_t e = pbase;
-      for (uint32_t q = 0; q < ng; ++q) {
-        pl.st[q] = e;
-        e += pl.ns[q] + pl.na[q];
-      }
+    const uint32_t before0 = x - n0 - n1, before1 = x - n1;  // superdroplets of the gridboxes before
+    // kept starts: s_q = max(b_q, end of q - 1, pbase), so s_q - before_q is the running maximum of
+    // b_i - before_i and pbase
+    const int64_t d0 = q0 < ng ? (int64_t)pl.b[q0] - before0 : INT64_MIN;
+    const int64_t d1 = q1 < ng ? (int64_t)pl.b[q1] - before1 : INT64_MIN;
+    int64_t m = max(d0, d1);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t y = __shfl_up_sync(0xFFFFFFFFu, m, o);
+      if ((int)lane >= o) m = max(m, y);
     }
-    for (uint32_t q = 0; q < ng; ++q)
-      pl.rw[q] = (!keep || pl.ns[q] != pl.oc[q] || pl.na[q] != 0 || pl.st[q] != pl.b[q]) ? 1 : 0;
+    const int64_t up = __shfl_up_sync(0xFFFFFFFFu, m, 1);
+    const int64_t m0 = max(max(lane ? up : INT64_MIN, d0), (int64_t)pbase);
+    const int64_t m1 = max(m0, d1);
+    const int64_t end = __shfl_sync(0xFFFFFFFFu, m1 + before1 + n1, 31);
+    const bool kept = keep && end <= (int64_t)pend;
+    const uint32_t s0 = kept ? (uint32_t)(m0 + before0) : pbase + before0;
+    const uint32_t s1 = kept ? (uint32_t)(m1 + before1) : pbase + before1;
+    if (q0 < ng) {
+      pl.st[q0] = s0;
+      pl.rw[q0] = (!keep || pl.ns[q0] != pl.oc[q0] || pl.na[q0] != 0 || s0 != pl.b[q0]) ? 1 : 0;
+    }
+    if (q1 < ng) {
+      pl.st[q1] = s1;
+      pl.rw[q1] = (!keep || pl.ns[q1] != pl.oc[q1] || pl.na[q1] != 0 || s1 != pl.b[q1]) ? 1 : 0;
+    }
   }
   __syncthreads();
 }
@@ -285,7 +309,7 @@ __device__ void stage_page(const DevCtx& c, uint32_t p, const PagePlan& pl) {
 }
 
 // whether every touched page still fits its slots (else pg_ctr[1] = 1: repack)
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(PG_THREADS)
 k_pg_plan(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ mk,
           const uint32_t* __restrict__ mvp, const uint32_t* __restrict__ m_ptr) {
   __shared__ PagePlan pl;
@@ -303,7 +327,7 @@ k_pg_plan(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ mk,
 // (taken when one does; then dst is copied back). Every slot of the page outside its gridboxes'
 // new ranges is left a hole.
 template <bool REPACK>
-__global__ void __launch_bounds__(256, 4)  // (256) alone caps it at 32 registers, with spills
+__global__ void __launch_bounds__(PG_THREADS, 2)
 k_pg_write(const __grid_constant__ DevCtx c, Fields dst, const uint32_t* __restrict__ mk,
            const uint32_t* __restrict__ mvp, const uint32_t* __restrict__ m_ptr,
            const uint32_t* __restrict__ pnew) {
@@ -358,7 +382,7 @@ k_pg_write(const __grid_constant__ DevCtx c, Fields dst, const uint32_t* __restr
   }
 }
 // repack path: page sizes for the new starts (every page: its new count plus the slack)
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(PG_THREADS)
 k_pg_sizes_repack(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ mk,
                   const uint32_t* __restrict__ mvp, const uint32_t* __restrict__ m_ptr,
                   uint32_t* __restrict__ psize) {

@@ -84,6 +84,7 @@ struct DevCtx {
   // re-sort after motion (pages.cuh): mover flags then their exclusive scan (slots + 1); a full
   // sort's per-key first sorted positions (ngbxs + 2)
   uint32_t *mv_scan, *gstart_new;  // mv_scan: movers per 32 slots, scanned (exclusive)
+  uint32_t* mv_page;   // a mover's old page at its slot (OOB for a null one)
   uint32_t* mv_mask;   // the movers among each 32 slots, a bit each (k_motion)
   uint32_t* mv_tsums;  // the count scan's tile offsets (the scan's readers add them: mv_before)
   uint32_t* mv_total;  // [0] valid superdroplets that changed gridbox in this motion step, [1] its
@@ -343,6 +344,7 @@ __device__ __forceinline__ bool move_superdroplet(const DevCtx& c, uint32_t i, u
   if (g >= ng) {  // a null superdroplet left by collisions (out of the domain), or a free slot
     const bool hole = is_hole(c.sd, i);
     if (!incremental) keys[i] = hole ? ng + 1 : ng;
+    else if (!hole) c.mv_page[i] = OOB;
     return !hole;  // a null one moves to the out-of-domain store
   }
     const Where w{c.err, g, i};
@@ -466,6 +468,7 @@ __device__ __forceinline__ bool move_superdroplet(const DevCtx& c, uint32_t i, u
     if (!incremental) keys[i] = key;  // the incremental re-sort takes min(gbx, ngbxs) instead
     // a superdroplet that changes gridbox (or leaves the domain) moves in the re-sort
     const bool mover = key != g;
+    if (incremental && mover) c.mv_page[i] = g / PAGE_GBXS;
     {  // count them (warp-aggregated) for the choice of the next re-sort
       const unsigned am = __activemask();
       const unsigned bm = __ballot_sync(am, mover);
@@ -873,69 +876,10 @@ __global__ void k_condsolve(const __grid_constant__ DevCtx c, uint32_t n, const 
   }
 }
 
-// ---- SDMMonitor members: one thread per gridbox, sums in the superdroplets' order ----
-// calculate_massmoments / calculate_rainmassmoments (massmoments_observer.cpp:38-113)
-__device__ __forceinline__ void mon_moments(const DevCtx& c, uint32_t g, int rain,
-                                            unsigned long long& m0, float& m1, float& m2) {
-  const double rlim = 40e-6 / R0;
-  const uint32_t base = c.gstart[g], n = c.gcount[g];
-  unsigned long long a0 = 0;
-  float a1 = 0.0f, a2 = 0.0f;
-  for (uint32_t k = base; k < base + n; ++k) {
-    const double r = c.sd.r[k];
-    const unsigned long long x = c.sd.xi[k];
-    const bool binary = rain ? (r >= rlim) : true;
-    a0 += x * (unsigned long long)binary;
-    const double mass = sd_mass(r, c.sd.msol[k]);
-    const double xi = (double)x;
-    a1 += (float)(xi * mass * (double)binary);
-    a2 += (float)(xi * mass * mass * (double)binary);
-  }
-  m0 = a0;
-  m1 = a1;
-  m2 = a2;
-}
-// fetch_delta_massmoments (monitor_massmoments_change.hpp:99-121); which = 0 after
-// microphysics, 1 after motion; begin != 0: before_timestepping (moments become the baseline)
-__global__ void k_mon_mm(const __grid_constant__ DevCtx c, int which, int begin) {
-  const int mask = c.p.monitors;
-  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < c.ngbxs;
-       g += gridDim.x * blockDim.x) {
-    for (int rain = 0; rain < 2; ++rain) {
-      if (!begin && !(mask & (rain ? CLEO_MONITOR_RAINMASSMOMENTS : CLEO_MONITOR_MASSMOMENTS)))
-        continue;
-      unsigned long long m0;
-      float m1, m2;
-      mon_moments(c, g, rain, m0, m1, m2);
-      if (!begin) {
-        c.mm0[rain][which][g] += m0 - c.prev0[rain][g];
-        c.mm1[rain][which][g] += m1 - c.prev1[rain][g];
-        c.mm2[rain][which][g] += m2 - c.prev2[rain][g];
-      }
-      c.prev0[rain][g] = m0;
-      c.prev1[rain][g] = m1;
-      c.prev2[rain][g] = m2;
-    }
-  }
-}
-// the precipitation contributions of each gridbox's superdroplets, in their order (the
-// reference adds them one by one as it moves the gridbox's superdroplets)
-__global__ void k_mon_precip(const __grid_constant__ DevCtx c) {
-  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < c.ngbxs;
-       g += gridDim.x * blockDim.x) {
-    const uint32_t base = c.gstart[g], n = c.gcount[g];
-    double acc = c.precip[g];
-    for (uint32_t k = base; k < base + n; ++k) {
-      const double v = c.precip_c[k];
-      if (v > 0.0) acc += v;
-    }
-    c.precip[g] = acc;
-  }
-}
-
 }  // namespace
 
 #include "batched.cuh"
+#include "monitors.cuh"
 #include "onebox.cuh"
 
 namespace {
@@ -1099,6 +1043,18 @@ int grid_for(size_t n, int threads) {
   return (int)b;
 }
 
+// gridboxes of a warp in the kernels that sum them in order: 32, or as few as keep 32 warps per SM
+uint32_t seq_per(const cleo_b200_ctx* x) {
+  uint32_t per = 32;
+  while (per > 1 && x->d.ngbxs / per < (uint32_t)x->sms * 32) per /= 2;
+  return per;
+}
+// blocks of `threads` for those kernels
+int seq_grid(const cleo_b200_ctx* x, int threads) {
+  const uint32_t per = seq_per(x);
+  return grid_for(((size_t)x->d.ngbxs + per - 1) / per * 32, threads);
+}
+
 // blocks of k_cond_place for a list of up to n solves, whose count only the device knows
 int place_grid(size_t n, int sms) {
   const size_t b = (n + PLACE_ITEMS - 1) / PLACE_ITEMS;
@@ -1173,18 +1129,18 @@ int sort_incremental(cleo_b200_ctx* x) {
                          x->ntiles_max, RS_SMALL_MAX, 0xFFFFFFFFu, &x->launches);
   const uint32_t* mk = where == 0 ? x->keys[1] : d.scr_p;
   const uint32_t* mvp = where == 0 ? x->vals[1] : d.scr_j;
-  const int pgrid = 148 * 8;  // CTAs over the touched pages (persistent loop)
+  const int pgrid = 148 * 4;  // CTAs over the touched pages (persistent loop)
   Fields& cur = x->buf[x->cur];
   Fields& other = x->buf[1 - x->cur];
   // grid-stride kernels over the movers, whose count only the device knows: one wave of CTAs
   const int mgrid = 148 * 8;
   k_mv_place<<<mgrid, 256, 0, s>>>(d, cur, mk, mvp, x->mv_count);
-  k_pg_plan<<<pgrid, 256, 0, s>>>(d, mk, mvp, x->mv_count);
-  k_pg_write<false><<<pgrid, 256, 0, s>>>(d, cur, mk, mvp, x->mv_count, d.pstart);
+  k_pg_plan<<<pgrid, PG_THREADS, 0, s>>>(d, mk, mvp, x->mv_count);
+  k_pg_write<false><<<pgrid, PG_THREADS, 0, s>>>(d, cur, mk, mvp, x->mv_count, d.pstart);
   // the repack path: its kernels return at once unless k_pg_plan chose it
-  k_pg_sizes_repack<<<pgrid, 256, 0, s>>>(d, mk, mvp, x->mv_count, x->pstart_new);
+  k_pg_sizes_repack<<<pgrid, PG_THREADS, 0, s>>>(d, mk, mvp, x->mv_count, x->pstart_new);
   k_pg_scan<<<1, SCAN_THREADS, 0, s>>>(d, x->pstart_new);
-  k_pg_write<true><<<pgrid, 256, 0, s>>>(d, other, mk, mvp, x->mv_count, x->pstart_new);
+  k_pg_write<true><<<pgrid, PG_THREADS, 0, s>>>(d, other, mk, mvp, x->mv_count, x->pstart_new);
   k_pg_copy_back<<<mgrid, 256, 0, s>>>(d, other, x->pstart_new);
   k_pg_commit<<<grid_for((size_t)d.npages + 1, 256), 256, 0, s>>>(d, x->pstart_new, x->mv_count);
   x->launches += 8;
@@ -1202,12 +1158,13 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
   StageMark m(x, 2);
   const int gg = grid_for(d.ngbxs, 256);
   // warps of 32 gridboxes each
-  const int gw = grid_for(((size_t)d.ngbxs + 31) / 32 * 32, SEQ_THREADS);
+  const int gw = seq_grid(x, SEQ_THREADS);
+  const uint32_t per = seq_per(x);
   // qcond from the moved superdroplets: summed by the first condensation sub-step's commit when
   // it starts the step (pass A stores each droplet's condensate mass before its solve), else here
   const bool fuse_qcond = did_motion && on_step(d.p.condstep, t_sdm);
   if (did_motion && !fuse_qcond) {
-    k_b_qcond<<<gw, SEQ_THREADS, 0, s>>>(d);
+    k_b_qcond<<<gw, SEQ_THREADS, 0, s>>>(d, per);
     x->launches += 1;
   }
   b.qm = nullptr;
@@ -1268,9 +1225,12 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
       }
       // every gridbox's condensed mass summed in order, its state updated (the gridboxes of
       // more than SEQ_BIG superdroplets by a warp each)
-      k_b_commit<<<gw, SEQ_THREADS, 0, s>>>(d, bc);
-      k_b_commit_big<<<x->sms * 4, SEQ_THREADS, 0, s>>>(d, bc);
-      x->launches += 3;
+      if (per > 1) {
+        k_b_commit<<<gw, SEQ_THREADS, 0, s>>>(d, bc, per);
+        x->launches += 1;
+      }
+      k_b_commit_big<<<x->sms * 4, SEQ_THREADS, 0, s>>>(d, bc, per > 1 ? 0 : 1);
+      x->launches += 2;
     }
     if (coll && x->one_box) {  // the one gridbox's collision step over the whole GPU
       StageMark mk(x, 4);
@@ -1341,7 +1301,8 @@ int run_sdm_step(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next) {
   DevCtx& d = x->d;
   cudaStream_t s = x->stream;
   const bool did_motion = on_step(d.p.motionstep, t_sdm);
-  const int gg = grid_for(d.ngbxs, 256);
+  const int gw = seq_grid(x, SEQ_THREADS);
+  const uint32_t per = seq_per(x);
   const bool mon_mm =
       (d.p.monitors & (CLEO_MONITOR_MASSMOMENTS | CLEO_MONITOR_RAINMASSMOMENTS)) != 0;
   if (did_motion) {
@@ -1361,7 +1322,7 @@ int run_sdm_step(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next) {
       }
       x->report_recorded = true;
       if (d.p.monitors & CLEO_MONITOR_PRECIPITATION) {  // before the sort moves the droplets
-        k_mon_precip<<<gg, 256, 0, s>>>(d);
+        k_mon_precip<<<gw, SEQ_THREADS, 0, s>>>(d, per);
         x->launches += 1;
       }
     }
@@ -1369,7 +1330,7 @@ int run_sdm_step(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next) {
     const int rc = x->sort_full ? sort_current(x) : sort_incremental(x);
     if (rc) return rc;
     if (mon_mm) {  // monitor_motion (movesupersindomain.hpp:297)
-      k_mon_mm<<<gg, 256, 0, s>>>(d, 1, 0);
+      k_mon_mm<<<seq_grid(x, MON_THREADS), MON_THREADS, 0, s>>>(d, 1, 0, per);
       x->launches += 1;
     }
   }
@@ -1377,7 +1338,7 @@ int run_sdm_step(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next) {
   if (d.p.exec_mode == CLEO_EXEC_BATCHED) {
     const int rc = run_batched_micro(x, t_sdm, t_sdm_next, did_motion);
     if (rc == CLEO_OK && mon_mm) {  // monitor_microphysics (sdmmethods.hpp:76)
-      k_mon_mm<<<gg, 256, 0, s>>>(d, 0, 0);
+      k_mon_mm<<<seq_grid(x, MON_THREADS), MON_THREADS, 0, s>>>(d, 0, 0, per);
       x->launches += 1;
     }
     return rc;
@@ -1391,7 +1352,7 @@ int run_sdm_step(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next) {
     }
   }
   if (mon_mm) {
-    k_mon_mm<<<gg, 256, 0, s>>>(d, 0, 0);
+    k_mon_mm<<<seq_grid(x, MON_THREADS), MON_THREADS, 0, s>>>(d, 0, 0, per);
     x->launches += 1;
   }
   CUDA_TRY(cudaGetLastError());
@@ -1637,6 +1598,7 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   rc |= dalloc(x, &x->tile_sums, ((size_t)256 * x->ntiles_max + SCAN_TILE - 1) / SCAN_TILE + 1);
   rc |= dalloc(x, &d.mv_scan, ((size_t)cap + 31) / 32 + 1);
   rc |= dalloc(x, &d.mv_mask, ((size_t)cap + 31) / 32);
+  rc |= dalloc(x, &d.mv_page, cap);
   rc |= dalloc(x, &d.mv_total, 2);
   if (cudaHostAlloc(&x->h_motion, 2 * sizeof(uint32_t), cudaHostAllocMapped) != cudaSuccess ||
       cudaHostGetDevicePointer(&x->d_motion, x->h_motion, 0) != cudaSuccess ||
@@ -2266,7 +2228,7 @@ int cleo_b200_monitors_begin(cleo_b200_ctx* x) {
   const DevCtx& d = x->d;
   if (!d.precip) return CLEO_OK;  // no monitors selected
   const size_t ng = d.ngbxs ? d.ngbxs : 1;
-  k_mon_mm<<<grid_for(d.ngbxs, 256), 256, 0, x->stream>>>(d, 0, 1);
+  k_mon_mm<<<seq_grid(x, MON_THREADS), MON_THREADS, 0, x->stream>>>(d, 0, 1, seq_per(x));
   x->launches += 1;
   for (int r = 0; r < 2; ++r)
     for (int w = 0; w < 2; ++w) {
