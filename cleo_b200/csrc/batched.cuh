@@ -333,10 +333,10 @@ k_cond_place(const uint32_t* __restrict__ n_ptr, const uint32_t* __restrict__ lk
 
 // ---- pass A: superdrop_mass_change (condensation.cpp:98-112) up to two Newton iterations ----
 // Bound by issue (930 instructions a warp of droplets, 400 of them FP64) and by the loads at the head
-// of each solve. A resident grid walks the slots, so the blocks' class counts are few; the gridbox
-// index, behind which the gridbox's values wait, is loaded a slot ahead. (Copying the next slot's
-// eight values ahead into shared memory as well was slower, 281 us for 225 on 5 M superdroplets: a
-// warp's copies of one gridbox's value are 32 separate ones.)
+// of each solve; the gridbox index, behind which the gridbox's values wait, is loaded a slot ahead.
+// 226 us for 5 M superdroplets at 4 CTAs per SM, 276 at 3. (Copying the next slot's eight values
+// ahead into shared memory as well was slower, 281 us: a warp's copies of one gridbox's value are
+// 32 separate ones.)
 template <int MINB>
 __global__ void __launch_bounds__(256, MINB)
 k_cond_a(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b) {

@@ -476,8 +476,7 @@ __device__ __forceinline__ bool move_superdroplet(const DevCtx& c, uint32_t i, u
     }
     return mover;
 }
-// A resident grid walks the slots (so few blocks count down at the end); the gridbox index, behind
-// which the gridbox's twelve values wait, is loaded a slot ahead.
+// (Loading the gridbox index a slot ahead, or a resident grid, was slower: 778 us for 708 on 40 M.)
 constexpr int MOTION_THREADS = 256, MOTION_CTAS = 4;  // 64 registers: 15% faster than 80
 __global__ void __launch_bounds__(MOTION_THREADS, MOTION_CTAS)
 k_motion(const __grid_constant__ DevCtx c, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
@@ -490,16 +489,11 @@ k_motion(const __grid_constant__ DevCtx c, uint32_t* __restrict__ keys, uint32_t
     c.pg_ctr[0] = c.pg_ctr[1] = c.pg_ctr[2] = 0;
     c.pg_ctr[3] += 1;
   }
-  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
   // i0 is the same for the whole block, so every warp's lanes cover 32 consecutive slots together
-  uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x;
-  uint32_t g_next = i0 + threadIdx.x < n ? c.sd.gbx[i0 + threadIdx.x] : OOB;
-  for (; i0 < n; i0 += step) {
-    const uint32_t i = (uint32_t)i0 + threadIdx.x;
-    const uint32_t g = g_next;
-    g_next = i0 + step + threadIdx.x < n ? c.sd.gbx[i0 + step + threadIdx.x] : OOB;
+  for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
+    const uint32_t i = i0 + threadIdx.x;
     bool mover = false;
-    if (i < n) mover = move_superdroplet(c, i, g, keys, vals, incremental);
+    if (i < n) mover = move_superdroplet(c, i, c.sd.gbx[i], keys, vals, incremental);
     if (incremental) {  // the movers of the warp's 32 slots: a mask and its count
       const unsigned bm = __ballot_sync(0xFFFFFFFFu, mover);
       if ((threadIdx.x & 31) == 0 && i < n) {
@@ -1055,6 +1049,11 @@ int seq_grid(const cleo_b200_ctx* x, int threads) {
   return grid_for(((size_t)x->d.ngbxs + per - 1) / per * 32, threads);
 }
 
+// Most waves of blocks of the kernels over all slots that end with a block's atomics: their number
+// costs (15 us of 116 at 9472 blocks on 5 M superdroplets), a resident grid's uneven shares cost
+// more (1.85 ms for 1.65 on 40 M)
+constexpr int WAVES = 6;
+
 // blocks of k_cond_place for a list of up to n solves, whose count only the device knows
 int place_grid(size_t n, int sms) {
   const size_t b = (n + PLACE_ITEMS - 1) / PLACE_ITEMS;
@@ -1189,7 +1188,7 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
       k_b_thermo<<<gg, 256, 0, s>>>(d, b, subt == t_sdm && !x->one_box ? 1 : 0);
       x->launches += 1;
       const int block = x->cfg.cond_block, minb = x->cfg.cond_minb;
-      const int ga = std::min(x->sms * minb * (256 / block), (int)grid_for(d.slots, block));
+      const int ga = std::min(x->sms * minb * (256 / block) * WAVES, (int)grid_for(d.slots, block));
       if (minb == 5)
         k_cond_a<5><<<ga, block, 0, s>>>(d, bc);
       else if (minb == 4)
@@ -1309,7 +1308,7 @@ int run_sdm_step(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next) {
     {
       StageMark m(x, 0);
       const bool inc = !x->sort_full;
-      k_motion<<<std::min(x->sms * MOTION_CTAS, grid_for(d.slots, MOTION_THREADS)),
+      k_motion<<<std::min(x->sms * MOTION_CTAS * WAVES, grid_for(d.slots, MOTION_THREADS)),
                  MOTION_THREADS, 0, s>>>(d, x->keys[0], x->vals[0], x->d_motion, inc ? 1 : 0);
       x->launches += 1;
       {  // inside a captured step the record becomes an external event node of the graph
