@@ -48,17 +48,15 @@ constexpr uint32_t OB_NONE = 0xFFFFFFFFu;
 
 struct OneBox {
   uint32_t* J;      // swap draws, index s (1 .. n-1)
-  uint32_t* cnt;    // per value: bucket size, then (scanned) bucket start; n + 1 entries
-  uint32_t* fill;   // per value: placement cursor
-  uint32_t* bkt;    // bucket contents (swap indexes), n entries
-  uint32_t* first;  // per value
+  uint32_t* head;   // per value: its list of swap indexes; all empty between steps
   uint32_t* next;   // per swap index
   uint32_t* P;      // origin of shuffled position k
   uint32_t* vflag;  // 1 for a valid superdroplet at shuffled position q, scanned; n + 1 entries
-  uint32_t* tsums;  // the scans' tile totals
+  uint32_t* tsums;  // the scan's tile totals
+  // these three 0 between steps:
   uint32_t* nnull;  // nulls made by this sub-step's collisions
   uint32_t* ninv;   // superdroplets left with multiplicity 0 (the flags' zeros)
-  uint32_t* nstep;  // the gridbox's count at the step's start (for k_ob_commit)
+  uint32_t* done;   // finished blocks of k_ob_gather
 };
 
 }  // namespace

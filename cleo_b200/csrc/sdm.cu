@@ -1060,17 +1060,6 @@ int place_grid(size_t n, int sms) {
   return (int)std::min<size_t>(b ? b : 1, (size_t)sms * 8);
 }
 
-// exclusive scan of a[0, n) on the context's stream, in place, the total into a[n] (tsums: the
-// scan's tile totals, (n + SCAN_TILE) / SCAN_TILE + 1 words)
-void scan_u32(cleo_b200_ctx* x, uint32_t* a, uint32_t n, uint32_t* tsums) {
-  cudaStream_t s = x->stream;
-  const uint32_t nt = (uint32_t)(((uint64_t)n + SCAN_TILE - 1) / SCAN_TILE);
-  k_scan_tiles<<<nt ? nt : 1, SCAN_THREADS, 0, s>>>(a, a, n, tsums);
-  k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(tsums, nt ? nt : 1, a + n);
-  k_scan_add<<<(unsigned)((n + 255) / 256 + 1), 256, 0, s>>>(a, n, tsums);
-  x->launches += 3;
-}
-
 // Full re-sort (pages.cuh): stable radix sort of the current buffer's slots [0, nrange) by the
 // keys in keys[0] (gridbox, out of domain, free slot), then the in-domain superdroplets written
 // into the other buffer page by page with PAGE_SLACK free slots after each page, the gridboxes'
@@ -1179,6 +1168,7 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
   }
   uint32_t subt = t_sdm;
   int colls = 0;  // collision sub-steps so far
+  bool one_box_end = false;  // the one-gridbox collision kernels have advanced the time
   while (subt < t_sdm_next) {
     const bool cond = on_step(d.p.condstep, subt);
     const bool coll = on_step(d.p.collstep, subt);
@@ -1234,35 +1224,31 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
     if (coll && x->one_box) {  // the one gridbox's collision step over the whole GPU
       StageMark mk(x, 4);
       const OneBox& o = x->ob;
-      const int go = grid_for((size_t)d.slots + 1, 256);
-      // scans of n + 1 entries (entries past n unused): one block while the slots allow
-      const bool one_block = (uint64_t)d.slots + 1 <= OB_SCAN_MAX;
-      const auto scan = [&](uint32_t* a, const uint32_t* skip) {
-        if (one_block) {
-          k_ob_scan<<<1, SCAN_THREADS, 0, s>>>(d, a, skip);
-          x->launches += 1;
-        } else {
-          scan_u32(x, a, d.slots + 1, o.tsums);
-        }
-      };
+      const int go = grid_for((size_t)d.slots + 1, OB_THREADS);
       const bool front = d.slots <= OB_FRONT_MAX;
-      if (front) {  // draws, counting sort, chains and their walks in one block
+      if (front) {  // draws, lists, chains and their walks in one block
         k_ob_front<<<1, OB_FRONT_THREADS, ob_front_smem(d.slots), s>>>(d, b, o);
-        x->launches += 1;
       } else {
         k_ob_draw<<<go, 256, 0, s>>>(d, b, o);
-        x->launches += 1;
-        scan(o.cnt, nullptr);  // bucket starts
-        k_ob_place<<<go, 256, 0, s>>>(d, o);
         k_ob_chains<<<go, 256, 0, s>>>(d, o);
-        x->launches += 2;
+        x->launches += 1;
       }
       k_ob_pairs<<<go, 256, 0, s>>>(d, b, o, front ? 1 : 0);
-      x->launches += 1;
-      scan(o.vflag, o.ninv);  // valid ones before each shuffled position (none to count: left out)
-      k_ob_gather<<<go, 256, 0, s>>>(d, o);
-      k_ob_commit<<<go, 256, 0, s>>>(d, b, o);
-      x->launches += 2;
+      if (!front) {  // valid ones before each shuffled position (left out where all are valid)
+        const uint64_t m = (uint64_t)d.slots + 1;
+        const uint32_t nt = (uint32_t)((m + SCAN_TILE - 1) / SCAN_TILE);
+        k_scan_tiles<<<nt, SCAN_THREADS, 0, s>>>(o.vflag, o.vflag, m, o.tsums, o.ninv, 0);
+        k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(o.tsums, nt, nullptr, o.ninv, 0);
+        k_scan_add<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(o.vflag, m, o.tsums, o.ninv, 0);
+        x->launches += 3;
+      }
+      const uint32_t next_subt = min(next_step(d.p.condstep, subt), next_step(d.p.collstep, subt));
+      one_box_end = next_subt >= t_sdm_next;  // the step's last sub-step: the gather advances the time
+      k_ob_gather<<<go, OB_THREADS, 0, s>>>(d, b, o, x->buf[1 - x->cur], front ? 0 : 1,
+                                            one_box_end ? t_sdm_next - t_sdm : 0u);
+      x->launches += 3;
+      x->cur = 1 - x->cur;
+      d.sd = x->buf[x->cur];
     } else if (coll) {
       StageMark mk(x, 4);
       if (colls++ > 0) {  // (the step's first finds its counters reset by k_b_reset above)
@@ -1290,8 +1276,10 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
     }
     subt = min(next_step(d.p.condstep, subt), next_step(d.p.collstep, subt));
   }
-  k_b_advance_t<<<1, 1, 0, s>>>(b, t_sdm_next - t_sdm, x->one_box ? 1 : 0);
-  x->launches += 1;
+  if (!one_box_end) {
+    k_b_advance_t<<<1, 1, 0, s>>>(b, t_sdm_next - t_sdm, x->one_box ? 1 : 0);
+    x->launches += 1;
+  }
   CUDA_TRY(cudaGetLastError());
   return CLEO_OK;
 }
@@ -1572,12 +1560,11 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   rc |= dalloc(x, &x->qm_buf, cap);
   if (ng == 1) {  // one gridbox: its collisions by the whole GPU (onebox.cuh)
     OneBox& o = x->ob;
-    for (uint32_t** q : {&o.J, &o.cnt, &o.fill, &o.bkt, &o.first, &o.next, &o.P, &o.vflag})
-      rc |= dalloc(x, q, cap + 2);
+    for (uint32_t** q : {&o.J, &o.head, &o.next, &o.P, &o.vflag}) rc |= dalloc(x, q, cap + 2);
     rc |= dalloc(x, &o.tsums, (cap + 2 + SCAN_TILE - 1) / SCAN_TILE + 1);
     rc |= dalloc(x, &o.nnull, 1);
     rc |= dalloc(x, &o.ninv, 1);
-    rc |= dalloc(x, &o.nstep, 1);
+    rc |= dalloc(x, &o.done, 1);
     x->one_box = true;
   }
   rc |= dalloc(x, &x->bs.zres, cap);
@@ -1659,9 +1646,10 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   CUDA_TRY(cudaMemsetAsync(d.pg_flag, 0, (size_t)d.npages * 4, x->stream));
   CUDA_TRY(cudaMemsetAsync(d.pg_ctr, 0, 16, x->stream));
   CUDA_TRY(cudaMemsetAsync(d.mv_stamp, 0, (size_t)d.ngbxs * 4, x->stream));
-  if (x->one_box) {  // the one-box counts start at zero (k_ob_gather clears what a step used)
-    CUDA_TRY(cudaMemsetAsync(x->ob.cnt, 0, ((size_t)d.slots + 2) * 4, x->stream));
-    CUDA_TRY(cudaMemsetAsync(x->ob.fill, 0, ((size_t)d.slots + 2) * 4, x->stream));
+  if (x->one_box) {  // empty lists, zero counters (k_ob_gather leaves them so)
+    CUDA_TRY(cudaMemsetAsync(x->ob.head, 0xFF, ((size_t)d.slots + 2) * 4, x->stream));
+    for (uint32_t* q : {x->ob.nnull, x->ob.ninv, x->ob.done})
+      CUDA_TRY(cudaMemsetAsync(q, 0, 4, x->stream));
   }
   CUDA_TRY(cudaMemsetAsync(d.err, 0, sizeof(DevError), x->stream));
   CUDA_TRY(cudaFuncSetAttribute(k_micro, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MICRO_SMEM));
