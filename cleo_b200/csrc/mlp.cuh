@@ -70,13 +70,109 @@ struct Infer {
   uint32_t* err;          // device status word: the first cleo_status failure is kept
 };
 
-__device__ __forceinline__ float gelu(float x) {
+// GELU(x) = x Phi(x) from one exponential: with z = -|x| and Phi(z) = 2^P(z), it is max(x, 0) + z 2^P.
+// P, log2 of the normal distribution's lower tail, is smooth: degree 10, P(0) = -1, fitted by
+// weighted least squares towards the smallest error of z 2^P (Lawson's iteration, on [-6, 0]);
+// below, the leading term takes it on to where 2^P vanishes (the argument is kept above -64, so that
+// infinities end there too). Largest error of the function 2.5e-7 (at 4 to 5: the result's rounding),
+// where 0.5 x (1 + erf) reaches 4.9e-7 by the cancellation below -2 and the roundings above 2; below
+// 1 in magnitude both are within 8e-8. Without erff's branch, and in fused operations that also run
+// in pairs (f2).
+__host__ __device__ constexpr float gelu_c(int k) {
+  return k == 0   ? 1.1511040925979614f
+         : k == 1 ? -0.45922335982322693f
+         : k == 2 ? 0.05242446810007095f
+         : k == 3 ? 0.006904458627104759f
+         : k == 4 ? -5.2864765166305006e-05f
+         : k == 5 ? -0.0003158595645800233f
+         : k == 6 ? -9.065421909326687e-05f
+         : k == 7 ? -1.4130660929367878e-05f
+         : k == 8 ? -1.2294659654799034e-06f
+                  : -4.6487080851420615e-08f;
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// max(x, 0), and not a number for -infinity, as x Phi(x) has it
+__device__ __forceinline__ float relu(float x) { return __fmaf_rn(0.5f, fabsf(x), 0.5f * x); }
+__device__ __forceinline__ float lower_arg(float x) { return fmaxf(-fabsf(x), -64.0f); }
+__device__ __forceinline__ float lower_tail(float z) {  // Phi(z), z <= 0
+  float p = gelu_c(9);
+#pragma unroll
+  for (int k = 8; k >= 0; --k) p = __fmaf_rn(p, z, gelu_c(k));
+  return ex2(__fmaf_rn(p, z, -1.0f));
+}
+// the form the hidden layer is rounded to BF16 from
+__device__ __forceinline__ float gelu_erf(float x) {
   return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f));
 }
+__device__ __forceinline__ float gelu(float x) {
+  const float z = lower_arg(x);
+  return __fmaf_rn(z, lower_tail(z), relu(x));
+}
+// pairs of floats in a 64-bit register (the low half first): each half of an operation is the
+// scalar operation
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2_pack(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(f2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 gelu_f2(f2 x, f2& z) {  // z: the lower arguments
+  float x0, x1, p0, p1;
+  f2_unpack(x, x0, x1);
+  z = f2_pack(lower_arg(x0), lower_arg(x1));
+  const f2 half = f2_pack(0.5f, 0.5f), zero = f2_pack(-0.0f, -0.0f);
+  const f2 r = f2_fma(f2_pack(fabsf(x0), fabsf(x1)), half, f2_fma(x, half, zero));  // relu
+  f2 p = f2_pack(gelu_c(9), gelu_c(9));
+#pragma unroll
+  for (int k = 8; k >= 0; --k) p = f2_fma(p, z, f2_pack(gelu_c(k), gelu_c(k)));
+  p = f2_fma(p, z, f2_pack(-1.0f, -1.0f));
+  f2_unpack(p, p0, p1);
+  return f2_fma(z, f2_pack(ex2(p0), ex2(p1)), r);
+}
+__device__ __forceinline__ f2 gelu_f2(f2 x) {
+  f2 z;
+  return gelu_f2(x, z);
+}
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-  const uint32_t a = __bfloat16_as_ushort(__float2bfloat16_rn(lo));
-  const uint32_t b = __bfloat16_as_ushort(__float2bfloat16_rn(hi));
-  return a | (b << 16);
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ uint32_t pack_bf16x2(f2 v) {
+  float a, b;
+  f2_unpack(v, a, b);
+  return pack_bf16x2(a, b);
+}
+// BF16(gelu_erf(x)) of a pair: the two GELUs differ by less than 1.8e-7 |x| (over all finite
+// arguments; most of it is the cancellation in 1 + erf), so where the quick one's neighbours at that
+// distance round alike, gelu_erf rounds there too; else (one pair in some hundreds, more below -2)
+// it decides itself.
+__device__ __forceinline__ uint32_t gelu_bf16x2(f2 x) {
+  f2 z;
+  const f2 v = gelu_f2(x, z);
+  const uint32_t lo = pack_bf16x2(f2_fma(z, f2_pack(2.0e-7f, 2.0e-7f), v));
+  const uint32_t hi = pack_bf16x2(f2_fma(z, f2_pack(-2.0e-7f, -2.0e-7f), v));
+  if (lo == hi) return lo;
+  float x0, x1;
+  f2_unpack(x, x0, x1);
+  return pack_bf16x2(gelu_erf(x0), gelu_erf(x1));
 }
 __device__ __forceinline__ float bf16_round(float x) {
   return __bfloat162float(__float2bfloat16_rn(x));
@@ -109,12 +205,13 @@ __device__ __forceinline__ void normalise(const float* fw, float x[NIN]) {
 __device__ __forceinline__ float denormalise(const float* fw, float y) {
   return fw[FW_NORM + 14] + fw[FW_NORM + 15] * y;
 }
-// hidden unit k of layer 1 (FP32 accumulation over the BF16-rounded weights)
+// hidden unit k of layer 1 (FP32 accumulation over the BF16-rounded weights); the tensor-core
+// kernel's pairs of units round to the same BF16 values
 __device__ __forceinline__ float hidden1(const float* fw, const float x[NIN], int k) {
   float a = fw[FW_B1 + k];
 #pragma unroll
   for (int i = 0; i < NIN; ++i) a += fw[FW_W1 + k * NIN + i] * x[i];
-  return gelu(a);
+  return gelu_erf(a);
 }
 
 // ---- tcgen05 primitives (PTX ISA 8.6+, sm_100a) ----
@@ -213,7 +310,8 @@ __device__ __forceinline__ void tmem_wait_ld() {
 constexpr uint32_t SM_A = 0;
 constexpr uint32_t SM_B = SM_A + A_BYTES;                             // 16384
 constexpr uint32_t SM_FW = SM_B + W2_UMMA_BYTES;                      // 24576
-constexpr uint32_t SM_BAR = SM_FW + ((NFW * 4 + 15) / 16) * 16;       // 27216
+constexpr uint32_t SM_W1 = SM_FW + ((NFW * 4 + 15) / 16) * 16;        // 27216
+constexpr uint32_t SM_BAR = SM_W1 + NH / 2 * 8 * 8;                   // 29264
 constexpr uint32_t SM_TSLOT = SM_BAR + 8;
 constexpr uint32_t TC_SMEM = 32768;  // rounded up: at most 7 CTAs per SM, 448 of 512 TMEM columns
 // persistent grid of the tensor-core kernel: every SM's 7 resident CTAs (tile phases of different
@@ -222,7 +320,11 @@ constexpr uint32_t TC_GRID_MAX = 148u * 7u;
 static_assert(SM_TSLOT + 4 <= TC_SMEM, "tensor-core kernel shared memory");
 constexpr uint32_t MBAR_TRIES = 1u << 22;
 
-// One persistent CTA of 128 threads per tile of 128 samples; thread t owns sample row t.
+// One persistent CTA of 128 threads per tile of 128 samples; thread t owns sample row t. Layer 1 and
+// both GELUs run on pairs of units (layer 1's weights as pairs, seven and the bias to a pair of
+// units): bound by FP32 issue and the 128 exponentials of a sample, 4 M samples 756 us with scalar
+// GELUs by erff, now 515 (some 410 if the hidden layer took the quick GELU and fused products
+// unchecked, which moves some of its BF16 roundings).
 // IO supplies raw features (io.features(i, x)) and consumes the denormalised output
 // (io.store(i, t)).
 template <class IO>
@@ -231,12 +333,18 @@ __global__ void __launch_bounds__(128) k_mlp_tc(Infer w, IO io, uint32_t n) {
   uint8_t* sA = smem + SM_A;
   uint4* sB = reinterpret_cast<uint4*>(smem + SM_B);
   float* sF = reinterpret_cast<float*>(smem + SM_FW);
+  f2* sW1 = reinterpret_cast<f2*>(smem + SM_W1);  // [k / 2][8]
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + SM_BAR);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + SM_TSLOT);
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
 
   for (uint32_t i = tid; i < W2_UMMA_BYTES / 16; i += 128) sB[i] = w.w2_umma[i];
   for (uint32_t i = tid; i < (uint32_t)NFW; i += 128) sF[i] = w.fw[i];
+  for (uint32_t i = tid; i < (uint32_t)NH / 2 * 8; i += 128) {
+    const uint32_t k = i / 8 * 2, q = i % 8;
+    const uint32_t at = q < NIN ? FW_W1 + k * NIN + q : FW_B1 + k, step = q < NIN ? NIN : 1;
+    sW1[i] = f2_pack(w.fw[at], w.fw[at + step]);
+  }
   if (tid == 0) mbar_init(bar, 1);
   if (warp == 0) tmem_alloc(tslot, TMEM_COLS);
   fence_async_smem();
@@ -246,6 +354,10 @@ __global__ void __launch_bounds__(128) k_mlp_tc(Infer w, IO io, uint32_t n) {
   const uint32_t tmem = *tslot;
   const uint32_t a_addr = smem_u32(sA), b_addr = smem_u32(sB);
   uint32_t phase = 0;
+  // -0 as a number the compiler does not know: w x + nz is the rounded product, which it would
+  // otherwise join with the sum (it contracts a packed multiply and add even without -fmad)
+  const float nz1 = __fmul_rn(-0.0f, (float)gridDim.x);
+  const f2 nz = f2_pack(nz1, nz1);
 
   n = io.rows(n);  // an IO may hold its row count in device memory (the same for every thread)
   for (uint32_t tile = blockIdx.x; (size_t)tile * TILE_M < n; tile += gridDim.x) {
@@ -256,15 +368,29 @@ __global__ void __launch_bounds__(128) k_mlp_tc(Infer w, IO io, uint32_t n) {
     for (int q = 0; q < NIN; ++q) x[q] = 0.0f;
     if (valid) io.features(i, x);
     normalise(sF, x);
+    f2 xp[NIN];
+#pragma unroll
+    for (int q = 0; q < NIN; ++q) xp[q] = f2_pack(x[q], x[q]);
     // layer 1 -> BF16 A tile, one 16-byte row segment of a core matrix per K chunk
 #pragma unroll 1
     for (uint32_t kc = 0; kc < NH / 8; ++kc) {
-      uint4 v;
-      v.x = pack_bf16x2(hidden1(sF, x, kc * 8 + 0), hidden1(sF, x, kc * 8 + 1));
-      v.y = pack_bf16x2(hidden1(sF, x, kc * 8 + 2), hidden1(sF, x, kc * 8 + 3));
-      v.z = pack_bf16x2(hidden1(sF, x, kc * 8 + 4), hidden1(sF, x, kc * 8 + 5));
-      v.w = pack_bf16x2(hidden1(sF, x, kc * 8 + 6), hidden1(sF, x, kc * 8 + 7));
-      *reinterpret_cast<uint4*>(sA + (kc * 16 + (tid >> 3)) * 128 + (tid & 7) * 16) = v;
+      uint32_t h[4];
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) {
+        const ulonglong2* row = reinterpret_cast<const ulonglong2*>(sW1 + (kc * 4 + q) * 8);
+        const ulonglong2 w01 = row[0], w23 = row[1], w45 = row[2], w6b = row[3];
+        // products and sums rounded apart, as hidden1's
+        f2 a = f2_add(w6b.y, f2_fma(w01.x, xp[0], nz));
+        a = f2_add(a, f2_fma(w01.y, xp[1], nz));
+        a = f2_add(a, f2_fma(w23.x, xp[2], nz));
+        a = f2_add(a, f2_fma(w23.y, xp[3], nz));
+        a = f2_add(a, f2_fma(w45.x, xp[4], nz));
+        a = f2_add(a, f2_fma(w45.y, xp[5], nz));
+        a = f2_add(a, f2_fma(w6b.x, xp[6], nz));
+        h[q] = gelu_bf16x2(a);
+      }
+      *reinterpret_cast<uint4*>(sA + (kc * 16 + (tid >> 3)) * 128 + (tid & 7) * 16) =
+          make_uint4(h[0], h[1], h[2], h[3]);
     }
     fence_async_smem();
     __syncthreads();
@@ -284,18 +410,24 @@ __global__ void __launch_bounds__(128) k_mlp_tc(Infer w, IO io, uint32_t n) {
     }
     phase ^= 1u;
     tc_fence_after();
-    float y = sF[FW_B3];
+    f2 y2 = f2_pack(sF[FW_B3], 0.0f);
 #pragma unroll
     for (uint32_t c = 0; c < NH / 16; ++c) {
       float acc[16];
       tmem_ld16(tmem + ((warp * 32u) << 16) + c * 16u, acc);
       tmem_wait_ld();
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
+      for (int j = 0; j < 16; j += 4) {  // two pairs of units
         const int col = (int)c * 16 + j;
-        y += sF[FW_W3 + col] * gelu(acc[j] + sF[FW_B2 + col]);
+        const ulonglong2 b2 = *reinterpret_cast<const ulonglong2*>(sF + FW_B2 + col);
+        const ulonglong2 w3 = *reinterpret_cast<const ulonglong2*>(sF + FW_W3 + col);
+        y2 = f2_fma(w3.x, gelu_f2(f2_add(f2_pack(acc[j], acc[j + 1]), b2.x)), y2);
+        y2 = f2_fma(w3.y, gelu_f2(f2_add(f2_pack(acc[j + 2], acc[j + 3]), b2.y)), y2);
       }
     }
+    float y, y_odd;
+    f2_unpack(y2, y, y_odd);
+    y += y_odd;
     if (valid) io.store(i, denormalise(sF, y));
     tc_fence_before();
     __syncthreads();
