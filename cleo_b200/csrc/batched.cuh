@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(SEQ_THREADS) k_b_qcond(const __grid_constant__
 __global__ void k_b_thermo(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b,
                            int first) {
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid < 2 * COST_CLASSES) b.ccnt[tid] = 0;
+  if (tid < COST_CLASSES + COST_CURSORS) b.ccnt[tid] = 0;
   if (first && tid < 8) b.ctr[1 + tid] = 0;  // bucket counts and heads
   for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < c.ngbxs; g += gridDim.x * blockDim.x) {
     if (g == 0) b.ctr[0] = b.ctr[10] = 0;  // deferred solves, big gridboxes
@@ -265,6 +265,18 @@ __device__ __forceinline__ uint32_t cost_class(double delt, double mindelt) {
   const float f = ns >= 1.0 ? (ns <= 65535.0 ? (float)ns : 65536.0f) : 1.0f;
   return 1u + ((__float_as_uint(f) >> 21) - (127u << 2));  // 1 .. 65
 }
+// Class of the restart that continues from zres (resume_restart): class 0, or LONG_RESTART, which is
+// counted in class 0 and placed behind its others. Where the solute term governs g, an iterate below
+// the root grows by 5/3 an iteration (g / (z g') is -2/3 there), and two iterations from a droplet's
+// own size can end at the floor of 1e-8, some 30 iterations below. So the logarithm of r^2 / zres
+// tells their number: 1 to 9 more up to 2^4, 22 to 37 from 2^14, little between. All in one class, a
+// warp's lanes were at work in 12 of 32 of its iterations where a fifth of the restarts are long
+// (k_cond_b 764 us for 2.9 M solves, now 541). The exponent and leading bits are the logarithm
+// within 0.09; five classes by it were no better, and their counting cost k_cond_a 9%.
+__device__ __forceinline__ uint32_t restart_class(double r, double zres) {
+  const int lg = 2 * __double2hiint(r) - __double2hiint(zres) - (1023 << 20);
+  return zres > 0.0 && lg >= (4 << 20) ? LONG_RESTART : 0u;
+}
 // the appended solves counted per class, a block's in shared memory first; every thread of the block
 // calls these. The restarts, most of the solves at a tight tolerance, are counted a warp at a time in
 // a register (one shared atomic each ran 32 in a row: 50 us of 275 for 5 M superdroplets).
@@ -274,8 +286,9 @@ __device__ __forceinline__ void class_count_begin(uint32_t* cnt) {
 }
 __device__ __forceinline__ void class_count(uint32_t* cnt, uint32_t& restarts, bool defer,
                                             uint32_t cls) {
-  restarts += __popc(__ballot_sync(0xFFFFFFFFu, defer && cls == 0u));
-  if (defer && cls != 0u) atomicAdd(&cnt[cls], 1u);
+  const bool restart = cls == 0u || cls == LONG_RESTART;
+  restarts += __popc(__ballot_sync(0xFFFFFFFFu, defer && restart));
+  if (defer && !restart) atomicAdd(&cnt[cls], 1u);
 }
 __device__ __forceinline__ void class_count_end(uint32_t* cnt, uint32_t restarts,
                                                 uint32_t* total) {
@@ -284,7 +297,7 @@ __device__ __forceinline__ void class_count_end(uint32_t* cnt, uint32_t restarts
   for (uint32_t i = threadIdx.x; i < COST_CLASSES; i += blockDim.x)
     if (cnt[i]) atomicAdd(&total[i], cnt[i]);
 }
-// The deferred solves by class, restarts first. Only neighbouring lanes' costs matter to pass B
+// The deferred solves by class, restarts first (the long ones fill their part from its end). Only neighbouring lanes' costs matter to pass B
 // (and the restarts' place to the surrogate), not the order within a class, so blocks of
 // PLACE_ITEMS solves take their shares of each class with one atomic: one launch where a radix
 // sort of the 16-bit costs took eleven, which returned at once or not (about 16 us of a step), and
@@ -294,17 +307,18 @@ __global__ void __launch_bounds__(256)
 k_cond_place(const uint32_t* __restrict__ n_ptr, const uint32_t* __restrict__ lkeys,
              const uint32_t* __restrict__ lvals, uint32_t* __restrict__ ccnt,
              uint32_t* __restrict__ order) {
-  __shared__ uint32_t cnt[COST_CLASSES], start[COST_CLASSES], total[COST_CLASSES];
+  __shared__ uint32_t cnt[COST_CURSORS], start[COST_CURSORS], total[COST_CLASSES];
   const uint32_t nl = *n_ptr;
   constexpr uint32_t PER = PLACE_ITEMS / 256;
   if (threadIdx.x < COST_CLASSES) total[threadIdx.x] = ccnt[threadIdx.x];
   for (uint32_t i0 = blockIdx.x * PLACE_ITEMS; i0 < nl; i0 += gridDim.x * PLACE_ITEMS) {
-    class_count_begin(cnt);
+    if (threadIdx.x < COST_CURSORS) cnt[threadIdx.x] = 0;
+    __syncthreads();
     uint32_t cls[PER], val[PER], rank[PER];
 #pragma unroll
     for (uint32_t q = 0; q < PER; ++q) {
       const uint32_t i = i0 + q * 256 + threadIdx.x;
-      cls[q] = i < nl ? lkeys[i] : COST_CLASSES;
+      cls[q] = i < nl ? lkeys[i] : COST_CURSORS;
       val[q] = i < nl ? lvals[i] : 0u;
     }
 #pragma unroll
@@ -312,21 +326,24 @@ k_cond_place(const uint32_t* __restrict__ n_ptr, const uint32_t* __restrict__ lk
       const unsigned peers = __match_any_sync(0xFFFFFFFFu, cls[q]);
       const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
       uint32_t base = 0;
-      if (lane == leader && cls[q] < COST_CLASSES)
+      if (lane == leader && cls[q] < COST_CURSORS)
         base = atomicAdd(&cnt[cls[q]], (uint32_t)__popc(peers));
       rank[q] = __shfl_sync(0xFFFFFFFFu, base, leader) + __popc(peers & ((1u << lane) - 1u));
     }
     __syncthreads();
-    if (threadIdx.x < COST_CLASSES) {
+    if (threadIdx.x < COST_CURSORS) {
       const uint32_t m = cnt[threadIdx.x];
       uint32_t s = m ? atomicAdd(&ccnt[COST_CLASSES + threadIdx.x], m) : 0u;
-      for (uint32_t k = 0; k < threadIdx.x; ++k) s += total[k];
+      if (threadIdx.x == LONG_RESTART)
+        s = total[0] - s - m;
+      else
+        for (uint32_t k = 0; k < threadIdx.x; ++k) s += total[k];
       start[threadIdx.x] = s;
     }
     __syncthreads();
 #pragma unroll
     for (uint32_t q = 0; q < PER; ++q)
-      if (cls[q] < COST_CLASSES) order[start[cls[q]] + rank[q]] = val[q];
+      if (cls[q] < COST_CURSORS) order[start[cls[q]] + rank[q]] = val[q];
     __syncthreads();
   }
 }
@@ -371,6 +388,7 @@ k_cond_a(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch 
         double radius, zres;
         if (!two_iterations(cfg, o, p.cond_delt, r, z0, ni, radius, zres)) {
           defer = true;  // restart from z0 until converged (impliciteuler.cpp:136-140)
+          key = restart_class(r, zres);
           b.zres[i] = zres;
           b.ffv[i] = ffactor_fv;
         } else {

@@ -13,6 +13,8 @@ constexpr uint32_t MEDIUM_SMEM = 24 * (MEDIUM_MAX + 2) + 8 * MEDIUM_MAX;
 constexpr uint32_t FY_PARALLEL_MAX = 256;  // gridboxes up to this size shuffle in parallel
 constexpr int B_THREADS = 256;
 constexpr uint32_t COST_CLASSES = 66;  // restarts, 64 quarter-octaves of sub-steps, those at 2^16
+constexpr uint32_t LONG_RESTART = COST_CLASSES;  // restarts of many iterations, counted in class 0
+constexpr uint32_t COST_CURSORS = COST_CLASSES + 1;
 constexpr int B_WARPS = B_THREADS / 32;
 
 struct BatchScratch {
@@ -27,16 +29,16 @@ struct BatchScratch {
                      // condensation sub-step after motion also gives qcond (else null)
   double* zres;      // per deferred direct solve: pass A's iterate that pass B resumes from
   double* ffv;       // per deferred solve: pass A's diffusion factor over the ventilation factor
-  uint32_t* lkeys;   // cost classes of deferred solves (cost_class)
+  uint32_t* lkeys;   // cost classes of deferred solves (restart_class, cost_class)
   uint32_t* lvals;   // positions of deferred solves
-  uint32_t* ccnt;    // [COST_CLASSES] solves per class, then [COST_CLASSES] k_cond_place's cursors
+  uint32_t* ccnt;    // [COST_CLASSES] solves per class, then [COST_CURSORS] k_cond_place's cursors
   uint32_t* order;   // the deferred solves by class
   uint32_t* bucket;  // [4][ngbxs] gridbox lists per size bucket
   uint4* brec;       // [2][ngbxs] the warp kernel's buckets as {gridbox, start, count, RNG slot}
   uint32_t* perm[2];  // the shuffles of those buckets' gridboxes (k_b_perm): 16 and 32 words each
   uint32_t* slot;    // per gridbox RNG slot offset within the SDM step
   uint32_t* ctr;     // [0] deferred solves, [1..4] bucket counts, [5..8] bucket heads,
-                     // [9] restarts among the deferred solves, [10] big gridboxes (commit)
+                     // [10] big gridboxes (commit)
   uint32_t* big;     // gridboxes whose condensation commit takes a warp each (k_b_commit_big)
   uint32_t* tsdm;    // the SDM step's start time (keys the injected random numbers)
   uint32_t small_max;   // gridboxes with 1..small_max superdroplets: warp kernel (<= WARP_MAX)

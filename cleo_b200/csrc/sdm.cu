@@ -881,7 +881,8 @@ namespace {
 // Two-pass form of the batch solve (the batched schedule), as k_cond_a / k_cond_b do for the
 // SDM step: pass A finishes every direct solve that converges within its first two iterations
 // (or within the seeded attempt) and lists the rest, keyed by sub-step count; pass B solves the
-// listed ones by cost class (k_cond_place), so that neighbouring lanes carry similar work. Iterations spent in pass A on an abandoned seed are carried in niters_out.
+// listed ones by cost class (k_cond_place), so that neighbouring lanes carry similar work. Iterations
+// spent in pass A on an abandoned seed are carried in niters_out.
 __device__ __forceinline__ uint32_t cs_warp_append(uint32_t* ctr, bool flag) {
   const unsigned m = __ballot_sync(0xFFFFFFFFu, flag);
   uint32_t base = 0;
@@ -937,7 +938,8 @@ k_cs_a(const __grid_constant__ DevCtx c, uint32_t n, const double* __restrict__ 
           out[i] = max_dryradius(radius, msol[i]);
           if (niters_out) niters_out[i] = ni | (failed ? CLEO_NITERS_FAILED : 0u);
         } else {
-          defer = true;  // restart until converged (impliciteuler.cpp:136-140), key 0
+          defer = true;  // restart until converged (impliciteuler.cpp:136-140)
+          key = seeded ? 0u : restart_class(r, zr);
           // where pass B's restart continues; NaN after an abandoned seed (a full solve)
           zres[i] = seeded ? __longlong_as_double(0x7FF8000000000000ll) : zr;
         }
@@ -1572,7 +1574,7 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   rc |= dalloc(x, &x->bs.lkeys, cap);
   rc |= dalloc(x, &x->bs.lvals, cap);
   rc |= dalloc(x, &x->bs.order, cap);
-  rc |= dalloc(x, &x->bs.ccnt, 2 * COST_CLASSES);
+  rc |= dalloc(x, &x->bs.ccnt, COST_CLASSES + COST_CURSORS);
   rc |= dalloc(x, &x->bs.bucket, 4 * ng);
   rc |= dalloc(x, &x->bs.big, ng);
   rc |= dalloc(x, &x->bs.brec, 2 * ng);
@@ -2317,7 +2319,7 @@ int cleo_b200_condensation_solve(cleo_b200_ctx* x, size_t n, const double* d_rad
   }
   // two-pass form: scratch for the deferred list of up to n solves
   auto& cs = x->cs;
-  constexpr size_t CTR_BYTES = (1 + 2 * COST_CLASSES) * sizeof(uint32_t);
+  constexpr size_t CTR_BYTES = (1 + COST_CLASSES + COST_CURSORS) * sizeof(uint32_t);
   if (n > cs.cap) {
     CUDA_TRY(cudaStreamSynchronize(x->stream));
     x->free_cs();
