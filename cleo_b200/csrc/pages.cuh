@@ -73,6 +73,18 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* a, uint32_t 
   }
   return lo;
 }
+// the same by a whole warp, which probes 32 places of the range at once
+__device__ __forceinline__ uint32_t lower_bound_warp(const uint32_t* a, uint32_t n, uint32_t v) {
+  uint32_t lo = 0, len = n;
+  while (len > 0) {
+    const uint32_t step = (len + 31) / 32, end = ((threadIdx.x & 31) + 1) * step;
+    const unsigned below = __ballot_sync(0xFFFFFFFFu, end <= len && a[lo + end - 1] < v);
+    const uint32_t c = __popc(below);  // (ascending: the first c lanes)
+    lo += c * step;
+    len = (c + 1) * step <= len ? step - 1 : len - c * step;
+  }
+  return lo;
+}
 // the page whose slots hold position i: the last p with pstart[p] <= i
 __device__ __forceinline__ uint32_t page_of_slot(const DevCtx& c, uint32_t i) {
   const uint32_t q = lower_bound_u32(c.pstart, c.npages + 1, i + 1);  // first pstart > i
@@ -91,20 +103,31 @@ __global__ void k_keys_paged(const __grid_constant__ DevCtx c, uint32_t* __restr
 // gp[k] = first sorted position with key >= k, k = 0 .. ngbxs + 1 (findrefs.hpp:54-126). Every page
 // holds its superdroplets and PAGE_SLACK free slots, so the page starts follow from gp alone. The
 // out-of-domain store's old count goes to counters[3], where k_gather_paged appends.
+// WARP: a warp per boundary, whose lanes probe 32 places of the range at once: four dependent loads
+// where a thread's search has some 18, whose latency is the launch's time on a small domain (10 us on
+// 256 or 4096 gridboxes with the caches cold, now 5). Up to LB_WARP_MAX gridboxes, where all the
+// warps are on the GPU together; beyond, the threads' searches already hide one another's loads.
+constexpr uint32_t LB_WARP_MAX = 8192;
+template <bool WARP>
 __global__ void k_lower_bounds(const __grid_constant__ DevCtx c, const uint32_t* __restrict__ keys,
                                uint32_t* __restrict__ gp) {
   const uint32_t n = c.counters[0];
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < c.ngbxs + 2;
-       k += gridDim.x * blockDim.x) {
-    const uint32_t a = lower_bound_u32(keys, n, k);
-    gp[k] = a;
-    if (k % PAGE_GBXS == 0 && (k < c.ngbxs || k == 0))
-      c.pstart[k / PAGE_GBXS] = a + k / PAGE_GBXS * PAGE_SLACK;
+  const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
+  const bool writes = !WARP || (threadIdx.x & 31) == 0;
+  for (uint32_t k = WARP ? first >> 5 : first; k < c.ngbxs + 2; k += WARP ? all >> 5 : all) {
+    const uint32_t a = WARP ? lower_bound_warp(keys, n, k) : lower_bound_u32(keys, n, k);
+    if (writes) {
+      gp[k] = a;
+      if (k % PAGE_GBXS == 0 && (k < c.ngbxs || k == 0))
+        c.pstart[k / PAGE_GBXS] = a + k / PAGE_GBXS * PAGE_SLACK;
+    }
     if (k == c.ngbxs) {
-      c.pstart[c.npages] = a + c.npages * PAGE_SLACK;
-      const uint32_t out = lower_bound_u32(keys, n, k + 1) - a;
-      c.counters[3] = c.counters[2];
-      c.counters[2] += out;
+      const uint32_t end = WARP ? lower_bound_warp(keys, n, k + 1) : lower_bound_u32(keys, n, k + 1);
+      if (writes) {
+        c.pstart[c.npages] = a + c.npages * PAGE_SLACK;
+        c.counters[3] = c.counters[2];
+        c.counters[2] += end - a;
+      }
     }
   }
 }

@@ -1077,7 +1077,10 @@ int sort_current(cleo_b200_ctx* x) {
   Fields& src = x->buf[x->cur];
   Fields& dst = x->buf[1 - x->cur];
   uint32_t* gp = d.gstart_new;
-  k_lower_bounds<<<grid_for((size_t)d.ngbxs + 2, 256), 256, 0, s>>>(d, kin, gp);
+  if (d.ngbxs <= LB_WARP_MAX)
+    k_lower_bounds<true><<<grid_for(((size_t)d.ngbxs + 2) * 32, 256), 256, 0, s>>>(d, kin, gp);
+  else
+    k_lower_bounds<false><<<grid_for((size_t)d.ngbxs + 2, 256), 256, 0, s>>>(d, kin, gp);
   k_gather_paged<<<grid_for(d.slots, 256), 256, 0, s>>>(d, src, dst, kin, vin, gp);
   x->launches += 2;
   x->cur = 1 - x->cur;

@@ -80,6 +80,21 @@ k_rs_downsweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vi
   const uint64_t base = (uint64_t)tile * RS_TILE;
   if (base >= n || (small_n > 0 && n <= small_n)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // warp w owns the contiguous chunk [w*32*ITEMS, (w+1)*32*ITEMS) of the tile, read in rounds of
+  // 32 consecutive keys: rank order = array order. Few tiles (SELF) load them all first, ahead of
+  // the table: there a block's own latency counts, 16 loads one behind another's ranking else (16
+  // tiles, caches cold: 14.8 us a pass, now 9.5). Many tiles load them round by round (all first takes 93 registers for 80 and was slower, 80 us a pass
+  // for 50 on 6.6 M keys)
+  uint32_t kk[RS_ITEMS], vv[RS_ITEMS], rk[RS_ITEMS];
+  const uint64_t own = base + (uint64_t)warp * 32 * RS_ITEMS + lane;
+  if constexpr (SELF) {
+#pragma unroll
+    for (int j = 0; j < RS_ITEMS; ++j) {
+      const uint64_t idx = own + (uint64_t)j * 32;
+      kk[j] = idx < n ? min(kin[idx], cap) : 0u;
+      vv[j] = idx < n ? (vin ? vin[idx] : (uint32_t)idx) : 0u;
+    }
+  }
   for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) (&wcount[0][0])[i] = 0;
   if constexpr (SELF) {
     // digit d = thread: the tiles' counts of it before this one, and in all
@@ -126,16 +141,14 @@ k_rs_downsweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vi
   }
   __syncthreads();
   const unsigned lt = (1u << lane) - 1u;
-  uint32_t kk[RS_ITEMS], vv[RS_ITEMS], rk[RS_ITEMS];
-  // warp w owns the contiguous chunk [w*32*ITEMS, (w+1)*32*ITEMS) of the tile, read in rounds of
-  // 32 consecutive keys: rank order = array order (loading all of them first takes 93 registers for
-  // 80 and was slower where there are many tiles: 80 us a pass for 50 on 6.6 M keys)
 #pragma unroll
   for (int j = 0; j < RS_ITEMS; ++j) {
-    const uint64_t idx = base + (uint64_t)warp * 32 * RS_ITEMS + (uint64_t)j * 32 + lane;
+    const uint64_t idx = own + (uint64_t)j * 32;
     const bool valid = idx < n;
-    kk[j] = valid ? min(kin[idx], cap) : 0u;
-    vv[j] = valid ? (vin ? vin[idx] : (uint32_t)idx) : 0u;
+    if constexpr (!SELF) {
+      kk[j] = valid ? min(kin[idx], cap) : 0u;
+      vv[j] = valid ? (vin ? vin[idx] : (uint32_t)idx) : 0u;
+    }
     const uint32_t d = valid ? ((kk[j] >> shift) & 255u) : 256u;
     const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
     const int leader = __ffs(peers) - 1;
