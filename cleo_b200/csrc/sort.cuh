@@ -83,8 +83,8 @@ k_rs_downsweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vi
   // warp w owns the contiguous chunk [w*32*ITEMS, (w+1)*32*ITEMS) of the tile, read in rounds of
   // 32 consecutive keys: rank order = array order. Few tiles (SELF) load them all first, ahead of
   // the table: there a block's own latency counts, 16 loads one behind another's ranking else (16
-  // tiles, caches cold: 14.8 us a pass, now 9.5). Many tiles load them round by round (all first takes 93 registers for 80 and was slower, 80 us a pass
-  // for 50 on 6.6 M keys)
+  // tiles, caches cold: 14.8 us a pass, now 9.5). Many tiles load them round by round: all first
+  // takes more than 80 registers and was slower (80 us a pass for 50 on 6.6 M keys).
   uint32_t kk[RS_ITEMS], vv[RS_ITEMS], rk[RS_ITEMS];
   const uint64_t own = base + (uint64_t)warp * 32 * RS_ITEMS + lane;
   if constexpr (SELF) {
