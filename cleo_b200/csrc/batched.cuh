@@ -274,7 +274,7 @@ __device__ __forceinline__ uint32_t cost_class(double delt, double mindelt) {
 // (k_cond_b 764 us for 2.9 M solves, now 541). The exponent and leading bits are the logarithm
 // within 0.09; five classes by it were no better, and their counting cost k_cond_a 9%.
 __device__ __forceinline__ uint32_t restart_class(double r, double zres) {
-  const int lg = 2 * __double2hiint(r) - __double2hiint(zres) - (1023 << 20);
+  const int hr = __double2hiint(r), lg = (hr - (1023 << 20)) + (hr - __double2hiint(zres));
   return zres > 0.0 && lg >= (4 << 20) ? LONG_RESTART : 0u;
 }
 // the appended solves counted per class, a block's in shared memory first; every thread of the block
