@@ -323,7 +323,7 @@ constexpr uint32_t MBAR_TRIES = 1u << 22;
 // One persistent CTA of 128 threads per tile of 128 samples; thread t owns sample row t. Layer 1 and
 // both GELUs run on pairs of units (layer 1's weights as pairs, seven and the bias to a pair of
 // units): bound by FP32 issue and the 128 exponentials of a sample, 4 M samples 756 us with scalar
-// GELUs by erff, now 515 (some 410 if the hidden layer took the quick GELU and fused products
+// GELUs by erff, now 520 (some 410 if the hidden layer took the quick GELU and fused products
 // unchecked, which moves some of its BF16 roundings).
 // IO supplies raw features (io.features(i, x)) and consumes the denormalised output
 // (io.store(i, t)).

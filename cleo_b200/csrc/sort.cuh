@@ -185,8 +185,8 @@ k_rs_downsweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vi
 // RS_SMALL_MAX: `bits` key bits in 8-bit passes between (k0, v0) and (k1, v1), leaving the result
 // where the multi-tile passes would (in (k0, v0) after an even number of passes). Returns at once
 // for larger n, which the multi-tile passes sort, unless `any` is set: then it takes them too, tile
-// after tile (a caller that expects few and launches no other passes; about 12 us a tile of 16384
-// and pass). The first pass's values may be positions (v_first null), its keys capped.
+// after tile (a caller that expects few and launches no other passes). The first pass's values may be
+// positions (v_first null), its keys capped.
 constexpr int RS_SMALL_THREADS = 1024;
 constexpr int RS_SMALL_WARPS = RS_SMALL_THREADS / 32;
 constexpr uint32_t RS_SMALL_MAX = (uint32_t)RS_SMALL_THREADS * RS_ITEMS;  // 16384
