@@ -133,6 +133,12 @@ __global__ void k_mlp_stats(uint32_t n, const float* __restrict__ feats,
 // warps per scheduler, a quarter of the time shared-memory loads; 512 threads of 2 x 4 outputs
 // read more (half the time) and took 33 us a step. A CTA takes several tiles when there are more
 // than TR_BLOCKS_MAX, adding to the same registers, so the partial rows stay few.
+//
+// The kernels of consecutive steps are on the GPU together (launch_step): an update writes params
+// while the next gradient kernel waits, a gradient kernel writes partial and loss_partial while its
+// update waits. So no pointer to those carries __restrict__, which would say that nothing else
+// writes them while the kernel runs and allow loads through the read-only path or ahead of the
+// wait, and they are read from L2 (__ldcg), where the writer's stores are.
 __device__ __forceinline__ void fma4x4(float acc[4][4], const float4 a[4], const float4 b[4]) {
 #pragma unroll
   for (int r = 0; r < 4; ++r)
@@ -158,10 +164,10 @@ __device__ __forceinline__ void gelu_both(float a, float& h, float& d) {
   d = __fmaf_rn(a, 0.39894228040143268f * expf(-0.5f * a * a), cdf);
 }
 __global__ void __launch_bounds__(TR_T, 2)
-k_mlp_fwdbwd(const float* __restrict__ params, const float* __restrict__ norm,
+k_mlp_fwdbwd(const float* params, const float* __restrict__ norm,
              const float* __restrict__ feats, const float* __restrict__ target, uint32_t n,
              uint32_t count, uint64_t seed, uint32_t step, int random,
-             float* __restrict__ partial, float* __restrict__ loss_partial, float inv_count) {
+             float* partial, float* loss_partial, float inv_count) {
   extern __shared__ __align__(16) float sm[];
   float* W2 = sm;                    // [j][k]
   float* H1 = W2 + TR_S * TR_LD;     // hidden 1 after GELU, [sample][k]
@@ -199,14 +205,14 @@ k_mlp_fwdbwd(const float* __restrict__ params, const float* __restrict__ norm,
   gather(blockIdx.x);
   cudaGridDependencySynchronize();
   for (uint32_t i = t; i < (uint32_t)(NH * NH); i += TR_T)
-    W2[(i / NH) * TR_LD + i % NH] = params[OFF_W2 + i];
+    W2[(i / NH) * TR_LD + i % NH] = __ldcg(&params[OFF_W2 + i]);
   for (uint32_t i = t; i < (uint32_t)(NH * 8); i += TR_T)
-    W1[i] = (i & 7) < NIN ? params[OFF_W1 + (i >> 3) * NIN + (i & 7)] : params[OFF_B1 + (i >> 3)];
+    W1[i] = __ldcg(&params[(i & 7) < NIN ? OFF_W1 + (i >> 3) * NIN + (i & 7) : OFF_B1 + (i >> 3)]);
   if (t < NH) {
-    B2[t] = params[OFF_B2 + t];
-    W3[t] = params[OFF_W3 + t];
+    B2[t] = __ldcg(&params[OFF_B2 + t]);
+    W3[t] = __ldcg(&params[OFF_W3 + t]);
   }
-  const float b3 = params[OFF_B3];
+  const float b3 = __ldcg(&params[OFF_B3]);
   float gw2[4][4], gw1[2] = {0.0f, 0.0f}, gv = 0.0f, gb3 = 0.0f, loss = 0.0f;
 #pragma unroll
   for (int r = 0; r < 4; ++r)
@@ -393,11 +399,9 @@ k_mlp_fwdbwd(const float* __restrict__ params, const float* __restrict__ norm,
 // 64 rows; now 4.9 us for 128 rows).
 constexpr int AD_P = 32, AD_G = 16;
 __global__ void __launch_bounds__(AD_P * AD_G)
-k_mlp_adam(float* __restrict__ params, float* __restrict__ m,
-                           float* __restrict__ v, const float* __restrict__ partial,
-                           uint32_t nblk, float lr_eff, float eps_eff, float beta1, float beta2,
-                           int apply, float* __restrict__ grad_out,
-                           const float* __restrict__ loss_partial, float* __restrict__ loss_out) {
+k_mlp_adam(float* params, float* m, float* v, const float* partial, uint32_t nblk, float lr_eff,
+           float eps_eff, float beta1, float beta2, int apply, float* grad_out,
+           const float* loss_partial, float* loss_out) {
   __shared__ float sums[AD_G][AD_P];
   const uint32_t p = threadIdx.x % AD_P, grp = threadIdx.x / AD_P;
   const uint32_t i = blockIdx.x * AD_P + p;
@@ -406,13 +410,13 @@ k_mlp_adam(float* __restrict__ params, float* __restrict__ m,
   float g = 0.0f;
   if (i < (uint32_t)NPARAM) {
 #pragma unroll 8
-    for (uint32_t b = grp; b < nblk; b += AD_G) g += partial[(size_t)b * NPARAM + i];
+    for (uint32_t b = grp; b < nblk; b += AD_G) g += __ldcg(&partial[(size_t)b * NPARAM + i]);
   }
   sums[grp][p] = g;
   __syncthreads();
   if (grp == 1 && blockIdx.x == 0 && loss_out) {  // a warp: the blocks' losses
     float l = 0.0f;
-    for (uint32_t b = p; b < nblk; b += AD_P) l += loss_partial[b];
+    for (uint32_t b = p; b < nblk; b += AD_P) l += __ldcg(&loss_partial[b]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xFFFFFFFFu, l, o);
     if (p == 0) *loss_out = l;
@@ -422,11 +426,11 @@ k_mlp_adam(float* __restrict__ params, float* __restrict__ m,
   for (int q = 1; q < AD_G; ++q) g += sums[q][p];
   if (grad_out) grad_out[i] = g;
   if (!apply) return;
-  const float mi = beta1 * m[i] + (1.0f - beta1) * g;
-  const float vi = beta2 * v[i] + (1.0f - beta2) * g * g;
+  const float mi = beta1 * __ldcg(&m[i]) + (1.0f - beta1) * g;
+  const float vi = beta2 * __ldcg(&v[i]) + (1.0f - beta2) * g * g;
   m[i] = mi;
   v[i] = vi;
-  params[i] -= lr_eff * mi / (sqrtf(vi) + eps_eff);
+  params[i] = __ldcg(&params[i]) - lr_eff * mi / (sqrtf(vi) + eps_eff);
 }
 
 // BF16 inference copies of the master weights
