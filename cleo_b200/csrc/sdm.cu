@@ -142,7 +142,6 @@ struct cleo_b200_ctx {
   cudaEvent_t ev_report = nullptr;
   bool report_recorded = false;
   bool sort_full = false;
-  bool movers_few = false;  // the previous motion step's movers: the page re-sort's own sort
   bool last_sort_full = false;  // what the last re-sort after motion was (cleo_b200_resort_stats)
   int resort_policy = CLEO_RESORT_AUTO;
   int sms = 148;                // the device's SMs
@@ -1107,16 +1106,19 @@ int sort_incremental(cleo_b200_ctx* x) {
   k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(d.mv_tsums, nscan, nullptr);
   k_mv_list<<<grid_for(n1, 256), 256, 0, s>>>(d, x->keys[1], x->vals[1], x->mv_count);
   x->launches += 3;
-  // the movers stably by key: up to RS_SMALL_MAX in one block; more by the multi-tile passes, which
-  // are only launched (their kernels return at once when they are not needed, 1.3 us each) when
-  // the last step's movers were not few; a step that then has many all the same stays with the block
-  const bool few = x->movers_few;
+  // the movers stably by key: up to RS_SMALL_MAX in one block; more by the multi-tile passes, whose
+  // kernels return at once when they are not needed (1.3 us each). Only the device knows this step's
+  // movers, and any number may move in the step after new winds whatever the last one's, so the
+  // passes are left out only where the store holds no more than the block sorts. (Left out after
+  // steps of few movers, with the block taking any number tile after tile, 1.85 M movers of a first
+  // windy step took 6.7 ms for the 1.6 they take now; the passes' empty launches cost 10 to 20 us of
+  // a step, 1.7% on 2 M superdroplets.)
   k_rs_small<<<1, RS_SMALL_THREADS, 0, s>>>(x->keys[1], x->vals[1], x->keys[1], x->vals[1], d.scr_p,
                                             d.scr_j, nullptr, x->mv_count, 0, x->key_bits,
-                                            few ? 1 : 0, 0xFFFFFFFFu);
+                                            0xFFFFFFFFu);
   x->launches += 1;
   int where = (int)(x->key_bits / 8 & 1);
-  if (!few)
+  if (d.slots > RS_SMALL_MAX)
     where = radix_passes(s, x->keys[1], x->vals[1], x->keys[1], x->vals[1], d.scr_p, d.scr_j,
                          nullptr, x->mv_count, 0, x->key_bits, x->hist, x->tile_sums,
                          x->ntiles_max, RS_SMALL_MAX, 0xFFFFFFFFu, &x->launches);
@@ -1429,7 +1431,7 @@ int run_step_graphed(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next) {
   const cleo_b200_params& p = x->d.p;
   std::vector<uint32_t> sig;
   sig.push_back((uint32_t)x->cur);
-  sig.push_back((on_step(p.motionstep, t_sdm) ? 1u : 0u) | (x->sort_full ? 2u : (x->movers_few ? 4u : 0u)));
+  sig.push_back((on_step(p.motionstep, t_sdm) ? 1u : 0u) | (x->sort_full ? 2u : 0u));
   sig.push_back(t_sdm_next - t_sdm);
   for (uint32_t subt = t_sdm; subt < t_sdm_next;
        subt = min(next_step(p.condstep, subt), next_step(p.collstep, subt))) {
@@ -1956,7 +1958,6 @@ int cleo_b200_step(cleo_b200_ctx* x, uint32_t t_mdl, uint32_t t_next) {
       if (x->report_recorded) CUDA_TRY(cudaEventSynchronize(x->ev_report));
       const volatile uint32_t* hm = x->h_motion;
       const uint32_t movers = hm[0], nsd = hm[1];
-      x->movers_few = x->report_recorded && movers <= RS_SMALL_MAX / 2;
       x->sort_full = x->resort_policy == CLEO_RESORT_FULL ||
                      (x->resort_policy == CLEO_RESORT_AUTO &&
                       ((uint64_t)movers * 5 > (uint64_t)nsd || x->d.npages < (uint32_t)x->sms));

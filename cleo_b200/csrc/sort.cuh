@@ -184,21 +184,20 @@ k_rs_downsweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vi
 // The same stable LSD sort in one block of RS_SMALL_THREADS, for counts (on the device) up to
 // RS_SMALL_MAX: `bits` key bits in 8-bit passes between (k0, v0) and (k1, v1), leaving the result
 // where the multi-tile passes would (in (k0, v0) after an even number of passes). Returns at once
-// for larger n, which the multi-tile passes sort, unless `any` is set: then it takes them too, tile
-// after tile (a caller that expects few and launches no other passes). The first pass's values may be
-// positions (v_first null), its keys capped.
+// for larger n, which the multi-tile passes sort. The first pass's values may be positions (v_first
+// null), its keys capped.
 constexpr int RS_SMALL_THREADS = 1024;
 constexpr int RS_SMALL_WARPS = RS_SMALL_THREADS / 32;
 constexpr uint32_t RS_SMALL_MAX = (uint32_t)RS_SMALL_THREADS * RS_ITEMS;  // 16384
 __global__ void __launch_bounds__(RS_SMALL_THREADS)
 k_rs_small(const uint32_t* k_first, const uint32_t* v_first, uint32_t* k0, uint32_t* v0,
            uint32_t* k1, uint32_t* v1, uint32_t* v_last, const uint32_t* __restrict__ n_ptr,
-           uint32_t n_val, uint32_t bits, int any, uint32_t cap) {
+           uint32_t n_val, uint32_t bits, uint32_t cap) {
   __shared__ uint32_t wcount[RS_SMALL_WARPS][256];
   __shared__ uint32_t dbase[256];
   __shared__ uint32_t wsum[8];
   const uint32_t n = n_ptr ? *n_ptr : n_val;
-  if (n > RS_SMALL_MAX && !any) return;
+  if (n > RS_SMALL_MAX) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const uint32_t d = threadIdx.x;  // digit of the threads below 256
@@ -208,81 +207,69 @@ k_rs_small(const uint32_t* k_first, const uint32_t* v_first, uint32_t* k0, uint3
   for (uint32_t shift = 0; shift < bits; shift += 8) {
     const uint32_t* kin = shift == 0 ? k_first : K[cur];
     const uint32_t* vin = shift == 0 ? v_first : V[cur];
-    if (n > RS_SMALL_MAX) {  // the digits' counts over all tiles
-      if (d < 256) dbase[d] = 0;
-      __syncthreads();
-      for (uint32_t i = threadIdx.x; i < n; i += RS_SMALL_THREADS)
-        atomicAdd(&dbase[(min(kin[i], cap) >> shift) & 255u], 1u);
-      __syncthreads();
+    for (int i = threadIdx.x; i < RS_SMALL_WARPS * 256; i += RS_SMALL_THREADS)
+      (&wcount[0][0])[i] = 0;
+    __syncthreads();
+    uint32_t kk[RS_ITEMS], vv[RS_ITEMS], rk[RS_ITEMS];
+#pragma unroll
+    for (int j = 0; j < RS_ITEMS; ++j) {  // array order = rank order, as in k_rs_downsweep
+      const uint32_t idx = (uint32_t)warp * 32 * RS_ITEMS + (uint32_t)j * 32 + lane;
+      const bool valid = idx < n;
+      kk[j] = valid ? min(kin[idx], cap) : 0u;
+      vv[j] = valid ? (vin ? vin[idx] : idx) : 0u;
+      rk[j] = 0xFFFFFFFFu;
     }
-    for (uint32_t t0 = 0; t0 < n || t0 == 0; t0 += RS_SMALL_MAX) {
-      for (int i = threadIdx.x; i < RS_SMALL_WARPS * 256; i += RS_SMALL_THREADS)
-        (&wcount[0][0])[i] = 0;
-      __syncthreads();
-      uint32_t kk[RS_ITEMS], vv[RS_ITEMS], rk[RS_ITEMS];
 #pragma unroll
-      for (int j = 0; j < RS_ITEMS; ++j) {  // array order = rank order, as in k_rs_downsweep
-        const uint32_t idx = t0 + (uint32_t)warp * 32 * RS_ITEMS + (uint32_t)j * 32 + lane;
-        const bool valid = idx < n;
-        kk[j] = valid ? min(kin[idx], cap) : 0u;
-        vv[j] = valid ? (vin ? vin[idx] : idx) : 0u;
-        rk[j] = 0xFFFFFFFFu;
-      }
-#pragma unroll
-      for (int j = 0; j < RS_ITEMS; ++j) {
-        const bool valid = t0 + (uint32_t)warp * 32 * RS_ITEMS + (uint32_t)j * 32 + lane < n;
-        if (t0 + (uint32_t)warp * 32 * RS_ITEMS + (uint32_t)j * 32 >= n) continue;  // whole warp
-        const uint32_t dg = valid ? ((kk[j] >> shift) & 255u) : 256u;
-        const unsigned peers = __match_any_sync(0xFFFFFFFFu, dg);
-        const int leader = __ffs(peers) - 1;
-        uint32_t prev = 0;
-        if (valid) prev = wcount[warp][dg];
-        __syncwarp();
-        if (valid && lane == leader) wcount[warp][dg] = prev + __popc(peers);
-        __syncwarp();
-        if (valid) rk[j] = prev + __popc(peers & lt);
-      }
-      __syncthreads();
-      // the per-warp offsets of a digit, then (first tile) the exclusive scan of the digits' totals
-      // over the first 8 warps
-      uint32_t tot = 0, x = 0, all = 0;
-      if (d < 256) {
+    for (int j = 0; j < RS_ITEMS; ++j) {
+      const uint32_t first = (uint32_t)warp * 32 * RS_ITEMS + (uint32_t)j * 32;
+      if (first >= n) continue;  // whole warp
+      const bool valid = first + lane < n;
+      const uint32_t dg = valid ? ((kk[j] >> shift) & 255u) : 256u;
+      const unsigned peers = __match_any_sync(0xFFFFFFFFu, dg);
+      const int leader = __ffs(peers) - 1;
+      uint32_t prev = 0;
+      if (valid) prev = wcount[warp][dg];
+      __syncwarp();
+      if (valid && lane == leader) wcount[warp][dg] = prev + __popc(peers);
+      __syncwarp();
+      if (valid) rk[j] = prev + __popc(peers & lt);
+    }
+    __syncthreads();
+    // the per-warp offsets of a digit, then the exclusive scan of the digits' totals over the first
+    // 8 warps
+    uint32_t tot = 0, x = 0;
+    if (d < 256) {
 #pragma unroll 8
-        for (int w = 0; w < RS_SMALL_WARPS; ++w) {
-          const uint32_t c = wcount[w][d];
-          wcount[w][d] = tot;
-          tot += c;
-        }
-        all = n > RS_SMALL_MAX ? dbase[d] : tot;
-        x = all;
+      for (int w = 0; w < RS_SMALL_WARPS; ++w) {
+        const uint32_t c = wcount[w][d];
+        wcount[w][d] = tot;
+        tot += c;
+      }
+      x = tot;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-          if (lane >= o) x += y;
-        }
-        if (lane == 31) wsum[warp] = x;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
       }
-      __syncthreads();
-      if (d < 256 && t0 == 0) {
-        uint32_t before = 0;
-        for (int w = 0; w < warp; ++w) before += wsum[w];
-        dbase[d] = before + x - all;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int j = 0; j < RS_ITEMS; ++j) {
-        if (rk[j] != 0xFFFFFFFFu) {
-          const uint32_t dg = (kk[j] >> shift) & 255u;
-          const uint32_t pos = dbase[dg] + wcount[warp][dg] + rk[j];
-          K[1 - cur][pos] = kk[j];
-          (v_last && shift + 8 >= bits ? v_last : V[1 - cur])[pos] = vv[j];
-        }
-      }
-      __syncthreads();  // this tile's writes before the next pass reads them
-      if (d < 256) dbase[d] += tot;  // the next tile's digits follow
-      if (n <= RS_SMALL_MAX) break;
-      __syncthreads();
+      if (lane == 31) wsum[warp] = x;
     }
+    __syncthreads();
+    if (d < 256) {
+      uint32_t before = 0;
+      for (int w = 0; w < warp; ++w) before += wsum[w];
+      dbase[d] = before + x - tot;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < RS_ITEMS; ++j) {
+      if (rk[j] != 0xFFFFFFFFu) {
+        const uint32_t dg = (kk[j] >> shift) & 255u;
+        const uint32_t pos = dbase[dg] + wcount[warp][dg] + rk[j];
+        K[1 - cur][pos] = kk[j];
+        (v_last && shift + 8 >= bits ? v_last : V[1 - cur])[pos] = vv[j];
+      }
+    }
+    __syncthreads();  // this pass's writes before the next pass reads them
     cur ^= 1;
   }
 }

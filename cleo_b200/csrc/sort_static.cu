@@ -132,7 +132,7 @@ extern "C" int cleo_b200_sort_by_gridbox_static(const uint32_t* d_sdgbxindex, ui
   if (n <= cleo::RS_SMALL_MAX) {
     cleo::k_rs_small<<<1, cleo::RS_SMALL_THREADS, 0, s>>>(d_sdgbxindex, nullptr, keys[0], vals[0],
                                                           keys[1], vals[1], v_last, nullptr, n,
-                                                          key_bits, 0, ngbxs);
+                                                          key_bits, ngbxs);
     cur = (int)(passes & 1);
   } else {
     cur = cleo::radix_passes(s, d_sdgbxindex, nullptr, keys[0], vals[0], keys[1], vals[1], v_last,
