@@ -1424,6 +1424,10 @@ int run_tuning_step(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next) {
   return CLEO_OK;
 }
 
+// Captured steps kept: those of eight patterns of sub-steps from either buffer (a full sort, and in a
+// one-gridbox domain each collision sub-step, makes the other buffer the current one)
+constexpr size_t GRAPHS_MAX = 16;
+
 // The launch sequence of one batched SDM step as a CUDA graph: captured the first time a
 // signature is seen, replayed afterwards. The injected random numbers are keyed by the device
 // word bs.tsdm, so a replay needs no parameter update.
@@ -1447,7 +1451,10 @@ int run_step_graphed(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next) {
       return CLEO_OK;
     }
   }
-  if (x->graphs.size() >= 8) x->drop_graphs();
+  if (x->graphs.size() >= GRAPHS_MAX) {  // the oldest goes
+    cudaGraphExecDestroy(x->graphs.front().exec);
+    x->graphs.erase(x->graphs.begin());
+  }
   const int cur0 = x->cur;
   const unsigned long long l0 = x->launches;
   CUDA_TRY(cudaStreamBeginCapture(x->stream, cudaStreamCaptureModeThreadLocal));
