@@ -1590,8 +1590,13 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
   rc |= dalloc(x, &x->bs.bucket, 4 * ng);
   rc |= dalloc(x, &x->bs.big, ng);
   rc |= dalloc(x, &x->bs.brec, 2 * ng);
-  for (int q = 0; q < 2; ++q)  // whole blocks of 32 gridboxes
-    rc |= dalloc(x, &x->bs.perm[q], (ng + 31) / 32 * 32 * ((q == 0 ? SMALL_MAX : WARP_MAX) / 4));
+  if (params->exec_mode == CLEO_EXEC_BATCHED) {
+    // the shuffles of the warp kernel's gridboxes, whole blocks of 32: no more gridboxes hold a
+    // superdroplet, or more than SMALL_MAX of them, than the capacity allows
+    const size_t most[2] = {std::min(ng, capacity), std::min(ng, capacity / (SMALL_MAX + 1))};
+    rc |= dalloc(x, &x->bs.perm[0], (most[0] + 31) / 32 * 32 * (SMALL_MAX / 4));
+    rc |= dalloc(x, &x->bs.perm[1], (most[1] + 31) / 32 * 32 * (WARP_MAX / 4));
+  }
   rc |= dalloc(x, &x->bs.slot, ng);
   rc |= dalloc(x, &x->bs.ctr, 12);
   rc |= dalloc(x, &x->bs.tsdm, 1);
