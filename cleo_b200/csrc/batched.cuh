@@ -31,6 +31,8 @@
 // whatever the schedule.
 #pragma once
 
+#include "pair_bound.h"
+
 namespace {
 
 using mlp::fence_async_smem;
@@ -559,8 +561,8 @@ __global__ void __launch_bounds__(SEQ_THREADS) k_b_commit_big(const __grid_const
 // One pair (2jj, 2jj+1) of the shuffled gridbox, collisions.hpp:140-158, on the drops at indexes
 // a and bb of the staged arrays. Few pairs collide in a step: a collision needs prob >= 1 or
 // phi_coll < prob (coalescence_gamma's and breakup's own tests), so a pair whose first random
-// number is at least an upper bound of its probability, below 1, is left as it is without
-// evaluating the probability. The bound is single precision (pair_apart); it replaces three FP64
+// number is above an upper bound of its probability, below 1, is left as it is without
+// evaluating the probability. The bound is single precision (pair_bound.h); it replaces three FP64
 // divisions, and two correctly rounded powers per pair (Simmel's velocities, a kernel over all
 // superdroplets and 16 bytes of traffic for each before).
 static __device__ __noinline__ uint32_t collide_pair_exact(const cleo_b200_params& p,
@@ -588,40 +590,6 @@ static __device__ __noinline__ uint32_t collide_pair_exact(const cleo_b200_param
   sm[i2] = d2.msol;
   return nn;
 }
-// What the probabilities of a gridbox's pairs share, in single precision: scale_p DELT / VOLUME
-// and the kernel's constant, 0.5% up to cover every rounding of the bound.
-__device__ __forceinline__ float pair_bound_coef(const cleo_b200_params& p, uint32_t n,
-                                                 double VOLUME) {
-  const float pairs = (float)(n / 2);
-  float k;
-  if (p.coll_prob == CLEO_PROB_GOLOVIN)
-    k = (float)(1.5e3 * R0 * R0 * R0 * 4.0 / 3.0 * PI);
-  else if (p.coll_prob == CLEO_PROB_LONG)
-    k = (float)(PI * R0 * R0 * W0) * fabsf((float)p.coaleff);
-  else
-    k = fabsf((float)p.const_kernel);
-  return 1.005f * ((float)n * ((float)n - 1.0f)) / (2.0f * pairs) *
-         (k * (float)p.coll_delt / (float)VOLUME);
-}
-// Whether a pair surely does not collide: phi (at most the random number) >= an upper bound of
-// prob. Golovin: r1^3 + r2^3. Long: the collection efficiency (its 1 - k2 / rsmall with 1e-5 to
-// spare), the squared sum of the radii, and for the difference of the terminal velocities the
-// larger droplet's, at most 1.189e-4 r^2 m/s (Simmel's first branch, which the others, 0.06% above
-// it where they meet, stay below beyond) and 9.18. NaN and overflow fail the comparison.
-__device__ __forceinline__ bool pair_apart(const cleo_b200_params& p, float coef, float r1,
-                                           float r2, float xi, float phi) {
-  float k = 1.0f;
-  if (p.coll_prob == CLEO_PROB_LONG) {
-    const float rs = fminf(r1, r2), rb = fmaxf(r1, r2), rb2 = rb * rb, sum = r1 + r2;
-    const float k1 = (float)(4.5e4 * R0 * R0 * 100 * 100), k2 = (float)(3e-4 / R0 / 100);
-    float eff = fmaxf(k1 * rb2 * (1.00001f - __fdividef(k2, rs)), 0.001f);
-    if (!(rb < 49.9f)) eff = fmaxf(eff, 1.0f);
-    k = eff * (sum * sum) * fminf(1.189e-4f / (float)W0 * rb2, 9.18f / (float)W0);
-  } else if (p.coll_prob == CLEO_PROB_GOLOVIN) {
-    k = r1 * r1 * r1 + r2 * r2 * r2;
-  }
-  return phi >= coef * xi * k;
-}
 __device__ __forceinline__ uint32_t collide_pair(const cleo_b200_params& p, unsigned long long* sx,
                                                  double* sr, double* sm, uint32_t a, uint32_t bb,
                                                  uint32_t n, float coef, double VOLUME,
@@ -629,10 +597,7 @@ __device__ __forceinline__ uint32_t collide_pair(const cleo_b200_params& p, unsi
                                                  const Where& w) {
   const unsigned long long xa = sx[a], xb = sx[bb];
   const uint64_t u = cleo_rng_u64(key, slot_pairs + 2ull * jj);
-  // the random number's leading 24 bits, a lower bound of it
-  const float phi = (float)(uint32_t)(u >> 40) * 0x1p-24f;
-  if (pair_apart(p, coef, (float)sr[a], (float)sr[bb], __ull2float_ru(xa < xb ? xb : xa), phi))
-    return 0;
+  if (pair_apart(p, coef, (float)sr[a], (float)sr[bb], pair_xi(xa, xb), pair_phi(u))) return 0;
   const uint32_t npairs = n / 2;
   const double scale_p = (double)n * ((double)n - 1.0) / (2.0 * (double)npairs);
   return collide_pair_exact(p, sx, sr, sm, a, bb, scale_p, VOLUME, key, slot_pairs + 2ull * jj, w);
@@ -747,6 +712,7 @@ k_b_small(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch
   constexpr uint32_t WORDS = CAP / 4;  // words of a gridbox's permutation (bytes)
   static_assert(CAP % 32 == 0 && CAP <= 128, "a word of the permutation per lane");
   const uint32_t t_sdm = *b.tsdm;
+  const float bound_kernel = pair_bound_kernel(c.p);
   extern __shared__ __align__(16) unsigned char smem_small[];
   const cleo_b200_params& p = c.p;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -820,7 +786,7 @@ k_b_small(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch
     const uint64_t key = cleo_rng_key(p.seed, t_sdm, g);
     const uint64_t slot_pairs = (uint64_t)rec.w + (n - 1);
     const uint32_t npairs = n / 2;
-    const float coef = pair_bound_coef(p, n, VOLUME);
+    const float coef = pair_bound_coef(bound_kernel, n, VOLUME);
     uint32_t nnull = 0;
     for (uint32_t j0 = 0; j0 < npairs; j0 += 32) {  // positions 2jj, 2jj + 1: word jj / 2
       const uint32_t jj = j0 + lane;
@@ -958,6 +924,7 @@ template <bool LARGE>
 __global__ void __launch_bounds__(LARGE ? LARGE_THREADS : B_THREADS)
 k_b_cta(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b) {
   const uint32_t t_sdm = *b.tsdm;
+  const float bound_kernel = pair_bound_kernel(c.p);
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint32_t shw[40];
   __shared__ uint32_t s_item;
@@ -1047,7 +1014,7 @@ k_b_cta(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b
     const uint64_t slot_pairs = slot + (n >= 1 ? n - 1 : 0);
     const uint32_t npairs = n / 2;
     const double VOLUME = c.volume[g] * VOL0;
-    const float coef = pair_bound_coef(p, n, VOLUME);
+    const float coef = pair_bound_coef(bound_kernel, n, VOLUME);
     uint32_t nnull = 0;
     for (uint32_t jj = tid; jj < npairs; jj += NT) {
       const uint32_t a = P[2 * jj], bb = P[2 * jj + 1];

@@ -181,7 +181,7 @@ __global__ void k_ob_pairs(const __grid_constant__ DevCtx c, const __grid_consta
   const uint64_t key = cleo_rng_key(c.p.seed, *b.tsdm, 0);
   const uint64_t slot_pairs = (uint64_t)b.slot[0] + (n >= 1 ? n - 1 : 0);
   const double VOLUME = c.volume[0] * VOL0;
-  const float coef = pair_bound_coef(c.p, n, VOLUME);
+  const float coef = pair_bound_coef(pair_bound_kernel(c.p), n, VOLUME);
   uint32_t nnull = 0, ninv = 0;
   for (uint32_t jj = blockIdx.x * blockDim.x + threadIdx.x; jj <= npairs;
        jj += gridDim.x * blockDim.x) {
