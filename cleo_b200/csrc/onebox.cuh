@@ -84,7 +84,10 @@ __global__ void k_ob_chains(const __grid_constant__ DevCtx c, OneBox o) {
 // NEXT as 16-bit indexes. The origins P go to global memory, so k_ob_pairs reads them instead of
 // walking the chains in global memory.
 constexpr uint32_t OB_FRONT_THREADS = 1024;
-constexpr uint32_t OB_FRONT_MAX = 28000;
+// One block's time grows with the store, the separate kernels' hardly (a step of 8000, 12000, 15900,
+// 20000 and 27900 superdroplets: 28.8, 32.2, 36.8, 38.8 and 47.2 us by the one, 33.0, 34.7, 36.8,
+// 36.7 and 37.8 by the others), so the line lies where they meet.
+constexpr uint32_t OB_FRONT_MAX = 16000;
 constexpr size_t ob_front_smem(uint32_t slots) { return (size_t)slots * 8 + 16; }
 __global__ void __launch_bounds__(OB_FRONT_THREADS)
 k_ob_front(const __grid_constant__ DevCtx c, const __grid_constant__ BatchScratch b, OneBox o) {

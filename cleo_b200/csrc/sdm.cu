@@ -1715,7 +1715,7 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
     x->grid_medium = sms * (occ > 0 ? occ : 1);
     CUDA_TRY(cudaFuncSetAttribute(k_b_cta<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)LARGE_SMEM));
-    if (x->one_box && x->d.slots <= OB_FRONT_MAX)  // at most 219 KB of tables
+    if (x->one_box && x->d.slots <= OB_FRONT_MAX)  // at most 125 KB of tables
       CUDA_TRY(cudaFuncSetAttribute(k_ob_front, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)ob_front_smem(x->d.slots)));
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_b_cta<true>, LARGE_THREADS,
