@@ -1715,9 +1715,9 @@ int cleo_b200_create(const cleo_b200_params* params, const cleo_b200_grid* grid,
     x->grid_medium = sms * (occ > 0 ? occ : 1);
     CUDA_TRY(cudaFuncSetAttribute(k_b_cta<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)LARGE_SMEM));
-    if (x->one_box && x->d.slots <= OB_FRONT_MAX)  // at most 125 KB of tables
-      CUDA_TRY(cudaFuncSetAttribute(k_ob_front, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)ob_front_smem(x->d.slots)));
+    // (125 KB; the limit is the process's, not this context's: the largest store's, whoever is last)
+    CUDA_TRY(cudaFuncSetAttribute(k_ob_front, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)ob_front_smem(OB_FRONT_MAX)));
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_b_cta<true>, LARGE_THREADS,
                                                            LARGE_SMEM));
     x->grid_large = sms * (occ > 0 ? occ : 1);

@@ -57,3 +57,19 @@ def test_one_box_no_slower_below_a_line(lib, below, above):
                 t[0] += w["tstep"]
         return _fastest(steps, 9)
     assert step(below) < step(above) * 7 / 6
+
+
+def test_a_smaller_box_beside_a_larger_one(lib):
+    """Members of an ensemble in one process: a later, smaller one leaves the larger one's
+    shared-memory limit alone."""
+    w = [W.box_golovin(n_sd=n, seed=n) for n in (15000, 500)]
+    runs = [make_sdm(x, lib=lib) for x in w]
+    for k in range(2):
+        for x, s in zip(w, runs):
+            s.run_step(k * x["tstep"], (k + 1) * x["tstep"])
+    for x, s in zip(w, runs):
+        s.check()
+        o = make_sdm(x, lib=K.oracle_lib(cr=True), prefix="oc")
+        for k in range(2):
+            o.run_step(k * x["tstep"], (k + 1) * x["tstep"])
+        K.assert_identical_run(s, o, "ensemble")
