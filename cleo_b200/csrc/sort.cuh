@@ -24,6 +24,8 @@ constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
+// (A block that adds the table up itself reads 1 KB a tile: two passes over 64 tiles 60 us against 63,
+// over 98 tiles 66 against 62.)
 constexpr uint32_t RS_SELF_TILES = 64;
 constexpr uint32_t RS_RAW_SUMS = 64;
 

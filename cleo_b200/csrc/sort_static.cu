@@ -26,6 +26,7 @@ namespace {
 namespace {
 
 constexpr uint32_t SORT_STATIC_MAX = 1u << 20;  // superdroplets per call
+constexpr uint32_t SMALL_MAX = 2 * cleo::RS_TILE;  // sorted by one block (<= RS_SMALL_MAX)
 constexpr uint32_t TILES_MAX = (SORT_STATIC_MAX + cleo::RS_TILE - 1) / cleo::RS_TILE;
 constexpr uint32_t HIST_MAX = 256 * TILES_MAX;
 constexpr uint32_t SCAN_SUMS_MAX = (HIST_MAX + cleo::SCAN_TILE - 1) / cleo::SCAN_TILE + 1;
@@ -39,6 +40,7 @@ constexpr size_t OFF_SUMS = OFF_HIST + HIST_MAX;
 constexpr size_t SCRATCH_WORDS = OFF_SUMS + SCAN_SUMS_MAX + 64;
 constexpr size_t SCRATCH_BYTES = SCRATCH_WORDS * sizeof(uint32_t);
 static_assert(SCRATCH_BYTES < (17u << 20), "the static scratch stays under 17 MiB");
+static_assert(SMALL_MAX <= cleo::RS_SMALL_MAX, "what the one-block sort takes");
 
 // The scratch memory. In host code this name is only a stand-in for the device symbol: the host
 // uses the address returned by cudaGetSymbolAddress, never the name itself.
@@ -122,14 +124,16 @@ extern "C" int cleo_b200_sort_by_gridbox_static(const uint32_t* d_sdgbxindex, ui
   // The first pass reads the gridbox indices themselves (capped: out-of-domain keys share the last
   // bucket, sortsupers.hpp:44-48) and its positions, the last writes the caller's order. The host's
   // launches bound the call: 1,000,003 superdroplets on 32,768 gridboxes, 12 launches 78 us, now 7
-  // (52 us); up to RS_SMALL_MAX, one block sorts them in one launch.
+  // (52 us); up to two tiles, one block sorts them in one launch. (One call after another, on 200,000
+  // gridboxes, three passes: 4096, 8192 and 16384 superdroplets by the block 47, 60 and 96 us, by
+  // the tiles 58, 58 and 65; on 20,000, two passes, 37, 47 and 68 against 47, 47 and 44.)
   // (One pass that overwrites its own input goes through the scratch instead.)
   const uint32_t passes = key_bits / 8;
   const bool in_place = passes == 1 && d_order < d_sdgbxindex + n && d_sdgbxindex < d_order + n;
   uint32_t* v_last = in_place ? nullptr : d_order;
   unsigned long long launches = 0;
   int cur;
-  if (n <= cleo::RS_SMALL_MAX) {
+  if (n <= SMALL_MAX) {
     cleo::k_rs_small<<<1, cleo::RS_SMALL_THREADS, 0, s>>>(d_sdgbxindex, nullptr, keys[0], vals[0],
                                                           keys[1], vals[1], v_last, nullptr, n,
                                                           key_bits, ngbxs);

@@ -73,3 +73,35 @@ def test_a_smaller_box_beside_a_larger_one(lib):
         for k in range(2):
             o.run_step(k * x["tstep"], (k + 1) * x["tstep"])
         K.assert_identical_run(s, o, "ensemble")
+
+
+def _static_sort(lib, n, ngbxs):
+    import ctypes as C
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    keys = torch.randint(0, ngbxs + 2, (n,), dtype=torch.int32, device="cuda", generator=gen)
+    order = torch.empty_like(keys)
+
+    def call():
+        assert lib.cleo_b200_sort_by_gridbox_static(
+            C.c_void_p(keys.data_ptr()), n, ngbxs, C.c_void_p(order.data_ptr()), None,
+            C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    return call, keys, order
+
+
+@pytest.mark.parametrize("ngbxs", [200, 20000, 200000])
+@pytest.mark.parametrize("n", [8191, 8192, 8193, 16384, 16385])
+def test_static_sort_beside_its_line(lib, n, ngbxs):
+    import torch
+    call, keys, order = _static_sort(lib, n, ngbxs)
+    call()
+    expect = torch.sort(keys.clamp(max=ngbxs), stable=True)[1]
+    assert torch.equal(order.long(), expect)
+
+
+@pytest.mark.parametrize("below,above", [(8192, 8193), (16384, 16385)])
+def test_static_sort_no_slower_below_a_line(lib, below, above):
+    def sorts(n):
+        call = _static_sort(lib, n, 200000)[0]
+        return _fastest(lambda: [call() for _ in range(100)], 15)
+    assert sorts(below) < sorts(above) * 7 / 6
