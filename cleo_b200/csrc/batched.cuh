@@ -1,7 +1,7 @@
 // batched.cuh — the batched microphysics of one SDM step (exec_mode CLEO_EXEC_BATCHED).
 //
 // Same results as k_micro (one CTA per gridbox), scheduled for B200 occupancy:
-//   k_b_qcond      warp per 32 gridboxes: qcond from the moved superdroplets (after the sort),
+//   k_b_qcond      warp per 1 to 32 gridboxes (seq_per): qcond from the moved superdroplets (after the sort),
 //                  their condensate masses added in order (warp_batch_sums)
 //   k_b_thermo     thread per gridbox: psat, supersaturation, diffusion factor, the droplets'
 //                  Kohler factors that depend on temperature alone
@@ -13,8 +13,9 @@
 //                  listed solves (the ones the reference guess did not settle in two iterations)
 //   k_cond_b       thread per listed solve, neighbouring lanes of similar cost, from the seed
 //                  where its residual beats the reference guess's
-//   k_b_commit     warp per 32 gridboxes: the condensed mass of each one's superdroplets added
-//                  in their order, their Newton iterations, and the state update
+//   k_b_commit     warp per 2 to 32 gridboxes: the condensed mass of each one's superdroplets
+//                  added in their order, their Newton iterations, and the state update
+//   k_b_commit_big the same, a warp each: large gridboxes, or all of a small domain's
 //   k_b_classify   gridboxes into size buckets (warp-aggregated atomics); the warp kernel's
 //                  buckets as records {gridbox, start, count, RNG slot}
 //   k_b_perm       thread per gridbox of the warp kernel's buckets: the Fisher-Yates shuffle
@@ -299,11 +300,11 @@ __device__ __forceinline__ void class_count_end(uint32_t* cnt, uint32_t restarts
   for (uint32_t i = threadIdx.x; i < COST_CLASSES; i += blockDim.x)
     if (cnt[i]) atomicAdd(&total[i], cnt[i]);
 }
-// The deferred solves by class, restarts first (the long ones fill their part from its end). Only neighbouring lanes' costs matter to pass B
-// (and the restarts' place to the surrogate), not the order within a class, so blocks of
-// PLACE_ITEMS solves take their shares of each class with one atomic: one launch where a radix
-// sort of the 16-bit costs took eleven, which returned at once or not (about 16 us of a step), and
-// 7 us where it sorted 400 thousand in 30.
+// The deferred solves by class, restarts first (the long ones fill their part from its end). Only
+// neighbouring lanes' costs matter to pass B (and the restarts' place to the surrogate), not the
+// order within a class, so blocks of PLACE_ITEMS solves take their shares of each class with one
+// atomic: one launch where a radix sort of the 16-bit costs took eleven, which returned at once or
+// not (about 16 us of a step), and 7 us where it sorted 400 thousand in 30.
 constexpr uint32_t PLACE_ITEMS = 1024;
 __global__ void __launch_bounds__(256)
 k_cond_place(const uint32_t* __restrict__ n_ptr, const uint32_t* __restrict__ lkeys,

@@ -1,7 +1,7 @@
 // monitors.cuh — SDMMonitor members: per-gridbox sums in the superdroplets' order.
 //
-// A warp takes up to 32 consecutive gridboxes (seq_per): it reads their contiguous range coalesced, a window at a
-// time, forms every superdroplet's terms once, and lane j adds gridbox g0 + j's from shared memory
+// A warp takes up to 32 consecutive gridboxes (seq_per): it reads their contiguous range coalesced,
+// a window at a time, forms every superdroplet's terms once, and lane j adds gridbox g0 + j's from shared memory
 // one after another, as the reference's loops do. A thread per gridbox reading its own range, for
 // all droplets and again for raindrops, took 147 us a call on 50 thousand gridboxes of 38 (twice a
 // step), now 45.

@@ -229,7 +229,7 @@ __device__ void plan_page(const DevCtx& c, uint32_t p, const uint32_t* mvp, Page
       const uint32_t k = k0 + lane;
       nst += __popc(__ballot_sync(0xFFFFFFFFu, k < n && c.sd.gbx[b + k] == g));
     }
-    // the movers into g (k_mv_runs), sorted by position: those before its old start lead
+    // the movers into g (k_mv_place), sorted by position: those before its old start lead
     const bool has = c.mv_stamp[g] == c.pg_ctr[3];
     const uint32_t lo = has ? c.mv_lo[g] : 0u, na = has ? c.mv_hi[g] - lo : 0u;
     uint32_t nl = 0;

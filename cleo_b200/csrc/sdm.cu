@@ -1152,7 +1152,7 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
   cudaStream_t s = x->stream;
   StageMark m(x, 2);
   const int gg = grid_for(d.ngbxs, 256);
-  // warps of 32 gridboxes each
+  // warps of `per` gridboxes each (seq_per)
   const int gw = seq_grid(x, SEQ_THREADS);
   const uint32_t per = seq_per(x);
   // qcond from the moved superdroplets: summed by the first condensation sub-step's commit when
@@ -1166,8 +1166,8 @@ int run_batched_micro(cleo_b200_ctx* x, uint32_t t_sdm, uint32_t t_sdm_next, boo
   BatchScratch bq = b;  // the first sub-step's scratch
   bq.qm = fuse_qcond ? x->qm_buf : nullptr;
   // every gridbox's RNG slot from 0 at the step's start, by the first condensation sub-step's
-  // k_b_thermo when it starts the step (a one-gridbox domain's was reset by the previous step's
-  // k_b_advance_t, or at creation)
+  // k_b_thermo when it starts the step (a one-gridbox domain's was reset at the previous step's end,
+  // by k_ob_gather where a collision sub-step ended it, else by k_b_advance_t, or at creation)
   const bool thermo_first = on_step(d.p.condstep, t_sdm);
   if (!x->one_box && !thermo_first) {
     k_b_reset<<<gg, 256, 0, s>>>(d, b, 1);
