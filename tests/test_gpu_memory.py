@@ -1,6 +1,8 @@
 """Device memory of a context: the shuffles' words (BatchScratch::perm) are sized by the gridboxes
 that can hold superdroplets, 64 bytes each and 128 for those of more than 64, and only the batched
 schedule has them."""
+import gc
+
 import pytest
 
 from cleo_b200 import abi
@@ -16,6 +18,7 @@ def _created(grid, capacity, mode):
     import torch
     assert torch.cuda.is_available(), "GPU tests need a CUDA device"
     p = make_params(condtstep=1.0, colltstep=1.0, motiontstep=1.0, exec_mode=mode)
+    gc.collect()  # contexts that earlier tests left behind
     before = torch.cuda.mem_get_info()[0]
     s = SDM(p, grid, capacity, lib=abi.load_library())
     used = before - torch.cuda.mem_get_info()[0]
